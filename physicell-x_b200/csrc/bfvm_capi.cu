@@ -401,6 +401,8 @@ int upload_coefficients(bfvm_ctx* c, const double* D, const double* decay) {
     c->dr_off[a] = dr_off[a];
     c->cu_off[a] = cu_off[a];
     c->conv_off[a] = conv_off[a];
+    const int* conv = reinterpret_cast<const int*>(host.data() + conv_off[a]);
+    c->conv_max[a] = *std::max_element(conv, conv + S);
   }
   BFVM_CUDA(cudaMemcpy(c->d_c1, c1.data(), S * sizeof(double), cudaMemcpyHostToDevice));
   // thomas_constant2 = decay; *= dt; /= 3 (BioFVM_solvers.cpp:208-209)
@@ -1161,6 +1163,7 @@ extern "C" int bfvm_set_wait_limit_ns(int device, unsigned long long ns) {
   DeviceGuard g(device);
   BFVM_CUDA(sweeps_set_wait_limit(ns));
   BFVM_CUDA(tmem_sweeps_set_wait_limit(ns));
+  BFVM_CUDA(pair_sweeps_set_wait_limit(ns));
   return BFVM_OK;
 }
 

@@ -33,6 +33,7 @@ struct bfvm_ctx {
   void* d_coef = nullptr;
   size_t dr_off[3] = {0, 0, 0}, cu_off[3] = {0, 0, 0};
   size_t conv_off[3] = {0, 0, 0};  // int [S] per axis: AxisCoefs::conv
+  int conv_max[3] = {0, 0, 0};     // the largest entry per axis
   void* d_c1 = nullptr;
   int screen = 0;              // SweepParams::screen of the 3-D sweeps (kScreenFast: short FP64 chain)
   int screen_exact = 0;        // 1 when no diffusion or decay rate is negative (the exactness screen applies)
@@ -228,6 +229,7 @@ inline SweepParams<T> make_params(bfvm_ctx* c, bool sources) {
     axes[a]->cu = reinterpret_cast<const CU*>(cb + c->cu_off[a]);
     axes[a]->npad = coef_pad(n_axis[a]);
     axes[a]->conv = reinterpret_cast<const int*>(cb + c->conv_off[a]);
+    axes[a]->conv_max = c->conv_max[a];
   }
   if (sources && c->n_agents > 0) {
     p.line_off = c->d_line_off;

@@ -60,6 +60,7 @@ struct AxisCoefs {
   // equal those of entry n - 2 (the factorization's fixed point), so that
   // the tensor-memory sweeps keep them in registers past it
   const int* conv;
+  int conv_max;  // the largest of them
 };
 
 // Rows of coefficient storage per line of n voxels: a y/z tile holds fewer
@@ -203,6 +204,11 @@ struct FieldMaps {
   // pyz_w = 0 when nx % 32 leaves nothing to pack (or is above 16).
   CUtensorMap py, pz;
   int pyz_w;
+  // the paired sweeps' forms of ry, rz, py, pz: chunks of 128 / elem_bytes rows
+  CUtensorMap qy, qz, qpy, qpz;
+  // the paired x sweep's: rows as xr, of the planes 1 .. nz - 2, plane 0 and
+  // plane nz - 1 (valid with xr_ok)
+  CUtensorMap qx[3];
 };
 
 // Host-side count of this library's kernel launches (bfvm_kernel_launches).
@@ -282,6 +288,15 @@ cudaError_t launch_tmem_yz_f32(const CUtensorMap& ring_map, const CUtensorMap& p
                                const SweepParams<float>& p, const SweepConfig& cfg, cudaStream_t st, bool* launched);
 cudaError_t launch_tmem_x_f32(const CUtensorMap& map, const SweepParams<float>& p, const SweepConfig& cfg,
                               cudaStream_t st, bool* launched);
+
+// The sweeps that run two tiles per warp (bfvm_pair_sweeps.cu), same
+// contract; map: FieldMaps::qx, or {qy, qpy, -} / {qz, qpz, -}.
+template <typename T, int AXIS>
+cudaError_t launch_pair(const CUtensorMap* const (&map)[3], int pw, const SweepParams<T>& p, const SweepConfig& cfg,
+                        cudaStream_t st, bool* launched);
+// TMEM rings of the single-tile sweep's plan for lines of n (0: none).
+int tmem_single_rings(int elem_bytes, int axis, int n, const SweepConfig& cfg);
+cudaError_t pair_sweeps_set_wait_limit(unsigned long long ns);
 
 // ---- batched engine: one fused launch per LOD step over many solves ------
 // Tiles are 32 lines (one warp) in every sweep of a batch.

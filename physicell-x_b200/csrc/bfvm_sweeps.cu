@@ -1443,6 +1443,14 @@ int encode_field_maps(FieldMaps* maps, void* f, int eb, int nx, int ny, int nz, 
   const cuuint32_t br[4] = {(cuuint32_t)(128 / eb), 32, 1, 1};
   maps->xr_ok = rc == 0 && rows < (1ull << 31) - 64 &&
                 encode_one(&maps->xr, f, eb, dr, sr, br, CU_TENSOR_MAP_SWIZZLE_128B, 3) == 0;
+  if (maps->xr_ok) {
+    const int k0[3] = {1, 0, nz - 1}, nk[3] = {nz - 2, 1, 1};
+    for (int q = 0; q < 3 && maps->xr_ok; ++q) {
+      const cuuint64_t dq[4] = {(cuuint64_t)nx, (cuuint64_t)ny * (nk[q] > 0 ? nk[q] : 1), (cuuint64_t)S, 1};
+      char* base = static_cast<char*>(f) + (nk[q] > 0 ? static_cast<size_t>(k0[q]) * ny * nxp * eb : 0);
+      maps->xr_ok = encode_one(&maps->qx[q], base, eb, dq, sr, br, CU_TENSOR_MAP_SWIZZLE_128B, 3) == 0;
+    }
+  }
   // the y/z sweeps' packed partial x tiles: a box of pw x by 32 / pw planes
   // by kRingRows rows along the line (the y map lists plane k before row j)
   maps->pyz_w = 0;
@@ -1456,6 +1464,22 @@ int encode_field_maps(FieldMaps* maps, void* f, int eb, int nx, int ny, int nz, 
     if (encode_one(&maps->py, f, eb, dpy, spy, bp, CU_TENSOR_MAP_SWIZZLE_NONE) == 0 &&
         encode_one(&maps->pz, f, eb, dims, strides, bp, CU_TENSOR_MAP_SWIZZLE_NONE) == 0)
       maps->pyz_w = w;
+  }
+  maps->qy = maps->ry;
+  maps->qz = maps->rz;
+  maps->qpy = maps->py;
+  maps->qpz = maps->pz;
+  if (rc == 0 && eb == 4) {
+    const cuuint32_t bqy[4] = {32, 32, 1, 1}, bqz[4] = {32, 1, 32, 1};
+    rc = encode_one(&maps->qy, f, eb, dims, strides, bqy, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc == 0) rc = encode_one(&maps->qz, f, eb, dims, strides, bqz, CU_TENSOR_MAP_SWIZZLE_NONE);
+    if (rc == 0 && maps->pyz_w > 0) {
+      const cuuint32_t bp[4] = {(cuuint32_t)maps->pyz_w, (cuuint32_t)(32 / maps->pyz_w), 32, 1};
+      const cuuint64_t dpy[4] = {(cuuint64_t)nx, (cuuint64_t)nz, (cuuint64_t)ny, (cuuint64_t)S};
+      const cuuint64_t spy[3] = {(cuuint64_t)nxp * ny * eb, (cuuint64_t)nxp * eb, (cuuint64_t)nxp * ny * nz * eb};
+      rc = encode_one(&maps->qpy, f, eb, dpy, spy, bp, CU_TENSOR_MAP_SWIZZLE_NONE);
+      if (rc == 0) rc = encode_one(&maps->qpz, f, eb, dims, strides, bp, CU_TENSOR_MAP_SWIZZLE_NONE);
+    }
   }
   return rc;
 }
@@ -1474,6 +1498,8 @@ cudaError_t launch_sweep_x(const FieldMaps& maps, const SweepParams<T>& p, const
     bool launched = false;
     cudaError_t e;
     if (maps.xr_ok) {
+      e = launch_pair<T, 0>({&maps.qx[0], &maps.qx[1], &maps.qx[2]}, 0, p, cfg, st, &launched);
+      if (e != cudaSuccess || launched) return e;
       if constexpr (sizeof(T) == 8)
         e = launch_tmem_x(maps.xr, p, cfg, st, &launched);
       else
@@ -1518,11 +1544,12 @@ constexpr long long kRingMinTilesPerCta = 8;
 
 template <typename T, int AXIS>
 static cudaError_t launch_yz_any(const CUtensorMap& map, const CUtensorMap& ring_map, const CUtensorMap& pmap, int pw,
-                                 const SweepParams<T>& p, const SweepConfig& cfg, cudaStream_t st) {
+                                 const CUtensorMap& qmap, const CUtensorMap& qpmap, const SweepParams<T>& p, const SweepConfig& cfg, cudaStream_t st) {
   const int n = (AXIS == 1) ? p.ny : p.nz;
   {
     bool launched = false;
-    cudaError_t e;
+    cudaError_t e = launch_pair<T, AXIS>({&qmap, &qpmap, &qpmap}, pw, p, cfg, st, &launched);
+    if (e != cudaSuccess || launched) return e;
     if constexpr (sizeof(T) == 8)
       e = launch_tmem_yz<AXIS>(ring_map, pmap, pw, p, cfg, st, &launched);
     else
@@ -1555,12 +1582,12 @@ static cudaError_t launch_yz_any(const CUtensorMap& map, const CUtensorMap& ring
 
 template <typename T>
 cudaError_t launch_sweep_y(const FieldMaps& maps, const SweepParams<T>& p, const SweepConfig& cfg, cudaStream_t st) {
-  return launch_yz_any<T, 1>(maps.y, maps.ry, maps.py, maps.pyz_w, p, cfg, st);
+  return launch_yz_any<T, 1>(maps.y, maps.ry, maps.py, maps.pyz_w, maps.qy, maps.qpy, p, cfg, st);
 }
 
 template <typename T>
 cudaError_t launch_sweep_z(const FieldMaps& maps, const SweepParams<T>& p, const SweepConfig& cfg, cudaStream_t st) {
-  return launch_yz_any<T, 2>(maps.z, maps.rz, maps.pz, maps.pyz_w, p, cfg, st);
+  return launch_yz_any<T, 2>(maps.z, maps.rz, maps.pz, maps.pyz_w, maps.qz, maps.qpz, p, cfg, st);
 }
 
 template cudaError_t launch_sweep_x<double>(const FieldMaps&, const SweepParams<double>&, const SweepConfig&,

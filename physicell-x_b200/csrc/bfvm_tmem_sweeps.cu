@@ -2187,6 +2187,16 @@ cudaError_t launch_tmem_x_f32(const CUtensorMap& map, const SweepParams<float>& 
   return cudaGetLastError();
 }
 
+int tmem_single_rings(int elem_bytes, int axis, int n, const SweepConfig& cfg) {
+  int ns = 0, nt = 0, kf = 0;
+  bool dr = false;
+  const bool on = elem_bytes == 8 ? (axis == 0 ? use_tmem_x(8, n, false, cfg, &ns, &nt, &kf)
+                                               : use_tmem_yz(8, n, cfg, &ns, &nt, &kf, &dr))
+                                  : (axis == 0 ? use_tmem_x_f32(4, n, false, cfg, &ns, &nt, &kf, &dr)
+                                               : use_tmem_yz_f32(4, n, cfg, &ns, &nt, &kf, &dr));
+  return on ? nt : 0;
+}
+
 cudaError_t tmem_sweeps_set_wait_limit(unsigned long long ns) { return set_module_wait_limit(ns); }
 
 }  // namespace bfvm
