@@ -411,7 +411,7 @@ int bfvm_get_sweep_schedule(bfvm_ctx* ctx, int* persistent);
  * sources and the pins are the same in both.  chain = 2: chain 1, except
  * that long y and z lines are solved by a partition
  * method (by default on lines of at least 512 voxels in FP64 and 448 in
- * FP32, where it is the faster one): eight warps share each 32-line tile,
+ * FP32 and where it is the faster one): eight warps share each 32-line tile,
  * each warp running both recurrences over one eighth of the line, joined
  * through segment products that the host forms in extended precision at
  * set-up.  Its results are

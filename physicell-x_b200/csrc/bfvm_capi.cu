@@ -109,10 +109,15 @@ void drop_step_graph(bfvm_ctx* c) {
 
 // Whether the y (axis 1) or z (axis 2) sweep runs partitioned: chain 2, a
 // line of at least part_min_line voxels, and a tile that fits one CTA.
-bool use_part(const bfvm_ctx* c, int axis) {
-  const int n = axis == 1 ? c->ny : c->nz;
-  return c->fp64_chain == 2 && n >= part_min_line(c) && (n + kRingRows - 1) / kRingRows <= kPartMaxChunks &&
-         part_smem_bytes(c->eb, n) <= 227 * 1024;
+// By default not where the sweep of two tiles per warp is the faster one.
+template <typename T, int AXIS>
+bool use_part(const bfvm_ctx* c, const SweepParams<T>& p) {
+  const int n = AXIS == 1 ? c->ny : c->nz;
+  if (c->fp64_chain != 2 || n < part_min_line(c) || (n + kRingRows - 1) / kRingRows > kPartMaxChunks ||
+      part_smem_bytes(c->eb, n) > 227 * 1024)
+    return false;
+  return c->part_min_line >= 0 || (sizeof(T) == 8 && n >= kPartMinLinePair64) ||
+         !pair_takes<T, AXIS>(c->maps.pyz_w, p, c->cfg);
 }
 
 // The launches of one LOD step on c->stream (also while capturing): the
@@ -132,12 +137,12 @@ int enqueue_step(bfvm_ctx* c, const SweepParams<T>& p, bool standalone, cudaEven
   if (ev) BFVM_CUDA(cudaEventRecord(ev[1], st));
   BFVM_CUDA(launch_sweep_x<T>(c->maps, p, c->cfg, st));
   if (ev) BFVM_CUDA(cudaEventRecord(ev[2], st));
-  if (use_part(c, 1))
+  if (use_part<T, 1>(c, p))
     BFVM_CUDA((launch_part<T, 1>(c->maps.ry, p, c->part[1], st)));
   else
     BFVM_CUDA(launch_sweep_y<T>(c->maps, p, c->cfg, st));
   if (ev) BFVM_CUDA(cudaEventRecord(ev[3], st));
-  if (use_part(c, 2))
+  if (use_part<T, 2>(c, p))
     BFVM_CUDA((launch_part<T, 2>(c->maps.rz, p, c->part[2], st)));
   else
     BFVM_CUDA(launch_sweep_z<T>(c->maps, p, c->cfg, st));
@@ -1075,34 +1080,48 @@ int bfvm_sample_agents(bfvm_ctx* c, double* out) {
 
 namespace {
 
-// Deterministic per-substrate sums: fixed block partials, then one block adds
-// the partials in order.
-template <typename T>
-__global__ void field_partial_sums(const T* __restrict__ f, int nx, int rows_per_s, int nxp, double* partial) {
+// Deterministic per-substrate sums: fixed block partials, then one block per
+// substrate adds them in a fixed tree.  A warp takes a row at a time, its
+// lanes along x (a 64-bit division per value and one thread adding all
+// partials had made the two launches SUM0 us at 160 x 200 x 120 x 3, now SUM1).
+constexpr int kSumParts = 1024;
+
+// The block's sum of every thread's value, in thread 0.
+__device__ __forceinline__ double block_sum_256(double acc) {
   __shared__ double red[256];
-  const int s = blockIdx.y;
-  const long long n = static_cast<long long>(rows_per_s) * nx;
-  double acc = 0.0;
-  for (long long q = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; q < n;
-       q += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long r = q / nx, i = q % nx;
-    acc += static_cast<double>(f[(static_cast<size_t>(s) * rows_per_s + r) * nxp + i]);
-  }
   red[threadIdx.x] = acc;
   __syncthreads();
   for (int o = 128; o > 0; o >>= 1) {
     if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[static_cast<size_t>(s) * gridDim.x + blockIdx.x] = red[0];
+  return red[0];
 }
 
-__global__ void field_final_sums(const double* partial, int nparts, int S, double* out) {
-  const int s = threadIdx.x;
-  if (s >= S) return;
+template <typename T>
+__global__ void __launch_bounds__(256) field_partial_sums(const T* __restrict__ f, int nx, int rows_per_s, int nxp,
+                                                          double* __restrict__ partial) {
+  const int s = blockIdx.y, lane = threadIdx.x & 31, warps = blockDim.x / 32;
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int r = blockIdx.x * warps + threadIdx.x / 32; r < rows_per_s; r += gridDim.x * warps) {
+    const T* row = f + (static_cast<size_t>(s) * rows_per_s + r) * nxp;
+    for (int i0 = lane; i0 < nx; i0 += 128) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (i0 + 32 * e < nx) acc[e] += static_cast<double>(row[i0 + 32 * e]);
+    }
+  }
+  const double sum = block_sum_256((acc[0] + acc[1]) + (acc[2] + acc[3]));
+  if (threadIdx.x == 0) partial[static_cast<size_t>(s) * gridDim.x + blockIdx.x] = sum;
+}
+
+__global__ void __launch_bounds__(256) field_final_sums(const double* __restrict__ partial, int nparts,
+                                                        double* __restrict__ out) {
+  const int s = blockIdx.x;
   double acc = 0.0;
-  for (int b = 0; b < nparts; ++b) acc += partial[static_cast<size_t>(s) * nparts + b];
-  out[s] = acc;
+  for (int b = threadIdx.x; b < nparts; b += 256) acc += partial[static_cast<size_t>(s) * nparts + b];
+  const double sum = block_sum_256(acc);
+  if (threadIdx.x == 0) out[s] = sum;
 }
 
 }  // namespace
@@ -1110,7 +1129,8 @@ __global__ void field_final_sums(const double* partial, int nparts, int S, doubl
 extern "C" int bfvm_field_sums(bfvm_ctx* c, double* out) {
   if (!c || !out) return BFVM_ERR_ARG;
   DeviceGuard g(c->device);
-  const int nparts = 1024;
+  const int rows = c->ny * c->nz;
+  const int nparts = std::min(kSumParts, (rows + 7) / 8);
   dim3 grid(nparts, c->S);
   double* partial = c->d_sums;
   double* res = c->d_sums + static_cast<size_t>(c->S) * nparts;
@@ -1121,7 +1141,7 @@ extern "C" int bfvm_field_sums(bfvm_ctx* c, double* out) {
     field_partial_sums<float><<<grid, 256, 0, c->stream>>>(static_cast<const float*>(c->f), c->nx, c->ny * c->nz,
                                                            c->nxp, partial);
   BFVM_CUDA(cudaGetLastError());
-  field_final_sums<<<1, 64, 0, c->stream>>>(partial, nparts, c->S, res);
+  field_final_sums<<<c->S, 256, 0, c->stream>>>(partial, nparts, res);
   BFVM_CUDA(cudaGetLastError());
   note_launches(2);
   BFVM_CUDA(cudaMemcpyAsync(out, res, sizeof(double) * c->S, cudaMemcpyDeviceToHost, c->stream));

@@ -246,9 +246,13 @@ size_t part_smem_bytes(int elem_bytes, int n_line);
 // B200, mean y/z sweep time on n^3 cubes, partitioned over serial short
 // chain: FP64 1.00 at n = 384 and 448, 0.94 at 512, 0.64 at 640; FP32 (the
 // serial sweeps with their tensor-memory rings) 1.21 at 288, 1.06 at 320,
-// 1.07 at 384, 0.93 at 448, 0.80 at 512, 0.65 at 640.
+// 1.07 at 384, 0.93 at 448, 0.80 at 512, 0.65 at 640.  Against the sweeps of
+// two tiles per warp, where those run, y sweep: FP64 1.07 at 512, 0.83 at 640
+// (hence kPartMinLinePair64 there); FP32 1.14 at 512, 1.26 at 640, 1.69 at 800,
+// 1.05 at 1000: never by default.
 constexpr int kPartMinLine64 = 512;
 constexpr int kPartMinLine32 = 448;
+constexpr int kPartMinLinePair64 = 576;
 template <typename T, int AXIS>
 cudaError_t launch_part(const CUtensorMap& map, const SweepParams<T>& p, const PartAxis& pa, cudaStream_t st);
 
@@ -294,6 +298,9 @@ cudaError_t launch_tmem_x_f32(const CUtensorMap& map, const SweepParams<float>& 
 template <typename T, int AXIS>
 cudaError_t launch_pair(const CUtensorMap* const (&map)[3], int pw, const SweepParams<T>& p, const SweepConfig& cfg,
                         cudaStream_t st, bool* launched);
+// Whether launch_pair would launch.
+template <typename T, int AXIS>
+bool pair_takes(int pw, const SweepParams<T>& p, const SweepConfig& cfg);
 // TMEM rings of the single-tile sweep's plan for lines of n (0: none).
 int tmem_single_rings(int elem_bytes, int axis, int n, const SweepConfig& cfg);
 cudaError_t pair_sweeps_set_wait_limit(unsigned long long ns);

@@ -946,17 +946,17 @@ static bool pair_wins(int n, const PairPlan& pl, long long tiles, int sms, bool 
   return pl.C >= 4 && n * 100 >= 93 * 32 * pl.C && (any_count || tiles >= 4 * rings);
 }
 
+// The plan of the launch for this solve; false where another form runs.
 template <typename T, int AXIS>
-cudaError_t launch_pair(const CUtensorMap* const (&map)[3], int pw, const SweepParams<T>& p, const SweepConfig& cfg,
-                        cudaStream_t st, bool* launched) {
-  *launched = false;
+static cudaError_t pair_choose(int pw, const SweepParams<T>& p, const SweepConfig& cfg, PairPlan* pl, long long* tiles,
+                               bool* takes) {
+  *takes = false;
   const int n = AXIS == 0 ? p.nx : (AXIS == 1 ? p.ny : p.nz);
   if (cfg.persistent < 1 || cfg.tmem == 0 || (AXIS == 0 ? cfg.x_lines : cfg.yz_tile) != 32 ||
       (AXIS == 0 && p.line_off != nullptr))
     return cudaSuccess;
   const AxisCoefs<T>& ac = AXIS == 0 ? p.ax : (AXIS == 1 ? p.ay : p.az);
-  PairPlan pl{};
-  if (!pair_plan<T, AXIS>(n, ac.conv ? ac.conv_max : n, pw, &pl)) return cudaSuccess;
+  if (!pair_plan<T, AXIS>(n, ac.conv ? ac.conv_max : n, pw, pl)) return cudaSuccess;
   long long per_s;
   if (AXIS == 0) {
     per_s = pair_x_tiles(p.ny, p.nz);
@@ -965,15 +965,34 @@ cudaError_t launch_pair(const CUtensorMap* const (&map)[3], int pw, const SweepP
     per_s = pw > 0 ? static_cast<long long>(p.nx / 32) * nm + (nm + P - 1) / P
                    : static_cast<long long>((p.nx + 31) / 32) * nm;
   }
-  const long long tiles = per_s * (p.s_hi - p.s_lo);
+  *tiles = per_s * (p.s_hi - p.s_lo);
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
-  if (!pair_wins<T>(n, pl, tiles, sms, cfg.persistent >= 2, tmem_single_rings(sizeof(T), AXIS, n, cfg)))
-    return cudaSuccess;
+  *takes = pair_wins<T>(n, *pl, *tiles, sms, cfg.persistent >= 2, tmem_single_rings(sizeof(T), AXIS, n, cfg));
   // few tiles: a tile or two per SM rather than full CTAs on some
-  if (tiles < static_cast<long long>(sms) * pl.rings) pl.rings = static_cast<int>((tiles + sms - 1) / sms);
+  if (*tiles < static_cast<long long>(sms) * pl->rings) pl->rings = static_cast<int>((*tiles + sms - 1) / sms);
+  return cudaSuccess;
+}
+
+template <typename T, int AXIS>
+bool pair_takes(int pw, const SweepParams<T>& p, const SweepConfig& cfg) {
+  PairPlan pl{};
+  long long tiles = 0;
+  bool takes = false;
+  return pair_choose<T, AXIS>(pw, p, cfg, &pl, &tiles, &takes) == cudaSuccess && takes;
+}
+
+template <typename T, int AXIS>
+cudaError_t launch_pair(const CUtensorMap* const (&map)[3], int pw, const SweepParams<T>& p, const SweepConfig& cfg,
+                        cudaStream_t st, bool* launched) {
+  *launched = false;
+  PairPlan pl{};
+  long long tiles = 0;
+  bool takes = false;
+  cudaError_t e = pair_choose<T, AXIS>(pw, p, cfg, &pl, &tiles, &takes);
+  if (e != cudaSuccess || !takes) return e;
   // more than half of an SM's, so that one CTA has the SM's tensor memory
   size_t smem = pair_smem(pl);
   if (smem < 116 * 1024) smem = 116 * 1024;
@@ -995,7 +1014,8 @@ cudaError_t launch_pair(const CUtensorMap* const (&map)[3], int pw, const SweepP
 
 #define BFVM_PAIR_INST(T, AXIS)                                                                                   \
   template cudaError_t launch_pair<T, AXIS>(const CUtensorMap* const (&)[3], int, const SweepParams<T>&,          \
-                                            const SweepConfig&, cudaStream_t, bool*);
+                                            const SweepConfig&, cudaStream_t, bool*);                            \
+  template bool pair_takes<T, AXIS>(int, const SweepParams<T>&, const SweepConfig&);
 BFVM_PAIR_INST(double, 0)
 BFVM_PAIR_INST(double, 1)
 BFVM_PAIR_INST(double, 2)
