@@ -152,10 +152,13 @@ int bfvm_agent_constants_device(int n, int S, double dt, double voxel_volume, co
  *  diffusion_decay_solver__constant_coefficients_LOD_3D_BLOCKING]
  * (BioFVM_microenvironment.cpp:1370-1384; BioFVM_solvers.cpp:102-780):
  * Dirichlet pin, x sweep, pin, y sweep, pin, z sweep, pin.  Asynchronous on
- * the solve's stream.  Runs of more than 16 steps replay a captured CUDA
- * graph of 16 steps (recaptured when the agents, tracking or launch settings
- * change), unless per-step timing is on or the caller is capturing the
- * solve's stream itself; the results are the same bits either way. */
+ * the solve's stream.  A small grid (up to 32 x 8 lines per SM and axis whose
+ * lines fit in shared memory, without internalization tracking, timing or
+ * launch settings of its own) runs up to 64 steps per launch; elsewhere runs
+ * of more than 16 steps replay a captured CUDA graph of 16 steps (recaptured
+ * when the agents, tracking or launch settings change), unless per-step timing
+ * is on or the caller is capturing the solve's stream itself; the results are
+ * the same bits either way. */
 int bfvm_step(bfvm_ctx* ctx, int nsteps, int flags);
 
 /* The source/sink stage alone (one call of
@@ -448,7 +451,8 @@ int bfvm_set_sweep_tmem(bfvm_ctx* ctx, int on);
 int bfvm_tmem_sweep_plan(int axis, int n_line, int tmem_level, int* smem_rings, int* tmem_rings, int* input_slots);
 
 /* Number of this library's kernels launched by the calls so far (counted on
- * the host at each launch). */
+ * the host at each launch; a launch that runs whole steps of a small grid
+ * counts once for every stage of theirs that it stands for). */
 long long bfvm_kernel_launches(void);
 
 /* Per-kernel timing, the device counterpart of the reference's per-step

@@ -224,6 +224,16 @@ template <typename T>
 int run_steps_plain(bfvm_ctx* c, int nsteps, bool sources) {
   const bool standalone = sources && c->n_agents > 0 && !c->cfg.fuse_sources;
   const SweepParams<T> p = make_params<T>(c, sources && !standalone);
+  {
+    // a small grid: the whole run in one launch, each stage counted as one
+    bool launched = false;
+    const int rc = run_resident<T>(c, make_params<T>(c, sources), NodeLines{}, false, nsteps, c->stream, &launched);
+    if (rc != BFVM_OK) return rc;
+    if (launched) {
+      note_launches(nsteps * (3 + (standalone ? 1 : 0)));
+      return BFVM_OK;
+    }
+  }
   // Runs of steps replay a captured graph of kGraphSteps steps (the same
   // launches, so the same bits), which removes most of the per-launch host
   // cost on small grids.  Not while timing per step, nor on a stream the
@@ -655,7 +665,7 @@ int bfvm_create(const bfvm_config* cfg, bfvm_ctx** out) {
   if (rc == BFVM_OK) rc = dalloc(c, reinterpret_cast<void**>(&c->d_active), S * sizeof(int));
   if (rc == BFVM_OK) rc = dalloc(c, reinterpret_cast<void**>(&c->d_faces), face_elems(c) * 8);
   if (rc == BFVM_OK) rc = dalloc(c, reinterpret_cast<void**>(&c->d_status), sizeof(int));
-  if (rc == BFVM_OK) rc = dalloc(c, reinterpret_cast<void**>(&c->d_tile_counter), 4 * sizeof(unsigned long long));
+  if (rc == BFVM_OK) rc = dalloc(c, reinterpret_cast<void**>(&c->d_tile_counter), 6 * sizeof(unsigned long long));
   if (rc == BFVM_OK) rc = dalloc(c, reinterpret_cast<void**>(&c->d_nvalid), sizeof(int));
   if (rc == BFVM_OK)
     rc = dalloc(c, reinterpret_cast<void**>(&c->d_line_off), sizeof(int) * (static_cast<size_t>(c->ny) * c->nz + 1));
@@ -667,7 +677,7 @@ int bfvm_create(const bfvm_config* cfg, bfvm_ctx** out) {
     return fail(BFVM_ERR_OOM);
   }
   if (cudaMemset(c->f, 0, c->field_bytes) != cudaSuccess || cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess ||
-      cudaMemset(c->d_tile_counter, 0, 4 * sizeof(unsigned long long)) != cudaSuccess)
+      cudaMemset(c->d_tile_counter, 0, 6 * sizeof(unsigned long long)) != cudaSuccess)
     return fail(BFVM_ERR_CUDA);
   // made here, not on first use, so that steps may run inside a caller's
   // stream capture of any mode
@@ -718,6 +728,7 @@ int bfvm_destroy(bfvm_ctx* c) {
   dfree(c, c->d_shift2d);
   dfree(c, c->d_zero_active);
   dfree(c, c->d_nodes);
+  dfree(c, c->d_node_lines);
   dfree(c, c->d_delta);
   dfree(c, c->d_mass);
   dfree(c, c->d_part);
@@ -1184,6 +1195,7 @@ extern "C" int bfvm_set_wait_limit_ns(int device, unsigned long long ns) {
   BFVM_CUDA(sweeps_set_wait_limit(ns));
   BFVM_CUDA(tmem_sweeps_set_wait_limit(ns));
   BFVM_CUDA(pair_sweeps_set_wait_limit(ns));
+  BFVM_CUDA(resident_set_wait_limit(ns));
   return BFVM_OK;
 }
 

@@ -47,7 +47,8 @@ struct bfvm_ctx {
   double* d_faces = nullptr;   // xface | yface | zface
   int* d_status = nullptr;
   int* h_status = nullptr;     // pinned host copy of d_status, read back in the same stream wait
-  unsigned long long* d_tile_counter = nullptr;  // [2] per substrate group: persistent sweeps' work counter
+  unsigned long long* d_tile_counter = nullptr;  // [2] per substrate group: persistent sweeps' work counter; [2]
+                                                 // the resident run's barrier
   double* d_sums = nullptr;    // partial sums + result
   bfvm::FieldMaps maps{};
   bfvm::SweepConfig cfg{};
@@ -84,6 +85,8 @@ struct bfvm_ctx {
   int* d_zero_active = nullptr; // [S] zeros: the 2-D sweeps pin no faces
   int n_nodes = 0;
   void* d_nodes = nullptr;      // long long offset [n] | double value [n][S] | uchar activation [n][S]
+  int node_most[2] = {0, 0};    // its NodeLines::most
+  int* d_node_lines = nullptr;  // nz == 1: order by y row [n] | by x column [n] | first [ny + 1] | first [nx + 1]
   // host-side mirrors
   std::vector<unsigned char> active;
   std::vector<double> faces;    // same layout as d_faces
@@ -188,6 +191,26 @@ inline void dfree(bfvm_ctx* c, void* p) {
   }
   cudaFree(p);
 }
+
+// A 2-D solve's Dirichlet nodes by line, for bfvm_resident.cu: offset in a
+// substrate plane, value and activation [n][S] of every node, and for x (0)
+// and y (1) lines the nodes in line order, first[axis][l] .. first[axis][l+1].
+struct NodeLines {
+  int n;
+  const long long* off;
+  const double* val;
+  const unsigned char* act;
+  const int* first[2];
+  const int* order[2];
+  int most[2];  // nodes of 32 lines (32 q ..) at most
+};
+// bfvm_resident.cu: nsteps whole steps of a small grid in one launch on st,
+// sources (p.line_off) and 2-D nodes included; *launched false where the solve
+// is too large for it or a launch setting asks for another form.
+template <typename T>
+int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, int nsteps, cudaStream_t st,
+                 bool* launched);
+cudaError_t resident_set_wait_limit(unsigned long long ns);
 
 inline AgentTrack track_params(const bfvm_ctx* c) {
   AgentTrack t{};

@@ -25,6 +25,7 @@
 // substrate and ny == 1 the two agree bit for bit (the oracle is checked
 // against the reference build there); elsewhere the reference has no
 // defined result to compare with.
+#include <algorithm>
 #include <cstring>
 
 #include "bfvm_ctx.h"
@@ -147,8 +148,8 @@ int ensure_2d(bfvm_ctx* c) {
 }
 
 template <typename T>
-SweepParams<T> make_params_2d(bfvm_ctx* c) {
-  SweepParams<T> p = make_params<T>(c, false);
+SweepParams<T> make_params_2d(bfvm_ctx* c, bool sources) {
+  SweepParams<T> p = make_params<T>(c, sources);
   using DR = typename Coef<T>::DR;
   using CU = typename Coef<T>::CU;
   const unsigned char* cb = static_cast<const unsigned char*>(c->d_coef2d);
@@ -166,9 +167,39 @@ SweepParams<T> make_params_2d(bfvm_ctx* c) {
   return p;
 }
 
+NodeLines node_lines(const bfvm_ctx* c) {
+  NodeLines nd{};
+  if (c->n_nodes == 0) return nd;
+  const size_t n = c->n_nodes;
+  const unsigned char* base = static_cast<const unsigned char*>(c->d_nodes);
+  const size_t a = ((sizeof(long long) * n + 255) / 256) * 256;
+  nd.n = c->n_nodes;
+  nd.off = reinterpret_cast<const long long*>(base);
+  nd.val = reinterpret_cast<const double*>(base + a);
+  nd.act = base + a + ((sizeof(double) * n * c->S + 255) / 256) * 256;
+  nd.order[0] = c->d_node_lines;
+  nd.order[1] = c->d_node_lines + n;
+  nd.first[0] = c->d_node_lines + 2 * n;
+  nd.first[1] = nd.first[0] + c->ny + 1;
+  for (int axis = 0; axis < 2; ++axis) nd.most[axis] = c->node_most[axis];
+  return nd;
+}
+
 template <typename T>
 int run_steps_2d(bfvm_ctx* c, int nsteps, bool sources) {
-  const SweepParams<T> p = make_params_2d<T>(c);
+  {
+    // a small grid: the whole run in one launch, each stage counted as one
+    const bool src = sources && c->n_agents > 0;
+    SweepParams<T> p = make_params_2d<T>(c, src);
+    bool launched = false;
+    const int rc = run_resident<T>(c, p, node_lines(c), true, nsteps, c->stream, &launched);
+    if (rc != BFVM_OK) return rc;
+    if (launched) {
+      note_launches(nsteps * (2 + (src ? 1 : 0) + (c->n_nodes > 0 ? 3 : 0)));
+      return BFVM_OK;
+    }
+  }
+  const SweepParams<T> p = make_params_2d<T>(c, false);
   for (int st = 0; st < nsteps; ++st) {
     if (sources) {
       const int rc = bfvm_apply_sources(c);
@@ -235,12 +266,42 @@ int bfvm_set_dirichlet_nodes(bfvm_ctx* c, int count, const int* voxel, const dou
   const int n = static_cast<int>(off.size());
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
   dfree(c, c->d_nodes);
+  dfree(c, c->d_node_lines);
   c->d_nodes = nullptr;
+  c->d_node_lines = nullptr;
   c->n_nodes = 0;
   if (n == 0) return BFVM_OK;
   const size_t bytes = nodes_bytes(n, S);
-  const int rc = dalloc(c, &c->d_nodes, bytes);
+  int rc = dalloc(c, &c->d_nodes, bytes);
   if (rc != BFVM_OK) return rc;
+  if (c->nz == 1) {  // the nodes by x line (row j) and by y line (column i)
+    std::vector<int> lines(2 * static_cast<size_t>(n) + c->ny + 1 + c->nx + 1);
+    int* first[2] = {lines.data() + 2 * static_cast<size_t>(n), lines.data() + 2 * static_cast<size_t>(n) + c->ny + 1};
+    for (int axis = 0; axis < 2; ++axis) {
+      const int m = axis == 0 ? c->ny : c->nx;
+      auto line_of = [&](int q) { return static_cast<int>(axis == 0 ? off[q] / c->nxp : off[q] % c->nxp); };
+      int* at = first[axis];
+      std::fill(at, at + m + 1, 0);
+      for (int q = 0; q < n; ++q) ++at[line_of(q) + 1];
+      for (int l = 0; l < m; ++l) at[l + 1] += at[l];
+      c->node_most[axis] = 0;
+      for (int l = 0; l < m; l += 32)
+        c->node_most[axis] = std::max(c->node_most[axis], at[std::min(m, l + 32)] - at[l]);
+      std::vector<int> next(at, at + m);
+      for (int q = 0; q < n; ++q) lines[static_cast<size_t>(axis) * n + next[line_of(q)]++] = q;
+    }
+    rc = dalloc(c, reinterpret_cast<void**>(&c->d_node_lines), lines.size() * sizeof(int));
+    if (rc == BFVM_OK && cudaMemcpy(c->d_node_lines, lines.data(), lines.size() * sizeof(int),
+                                    cudaMemcpyHostToDevice) != cudaSuccess)
+      rc = BFVM_ERR_CUDA;
+    if (rc != BFVM_OK) {
+      dfree(c, c->d_nodes);
+      dfree(c, c->d_node_lines);
+      c->d_nodes = nullptr;
+      c->d_node_lines = nullptr;
+      return rc;
+    }
+  }
   std::vector<unsigned char> host(bytes, 0);
   const size_t a = ((sizeof(long long) * n + 255) / 256) * 256;
   const size_t b = ((sizeof(double) * static_cast<size_t>(n) * S + 255) / 256) * 256;
