@@ -152,9 +152,9 @@ int bfvm_agent_constants_device(int n, int S, double dt, double voxel_volume, co
  *  diffusion_decay_solver__constant_coefficients_LOD_3D_BLOCKING]
  * (BioFVM_microenvironment.cpp:1370-1384; BioFVM_solvers.cpp:102-780):
  * Dirichlet pin, x sweep, pin, y sweep, pin, z sweep, pin.  Asynchronous on
- * the solve's stream.  A small grid (up to 32 x 8 lines per SM and axis whose
- * lines fit in shared memory, without internalization tracking, timing or
- * launch settings of its own) runs up to 64 steps per launch; elsewhere runs
+ * the solve's stream.  A grid that stays in the L2 and whose lines fit in shared
+ * memory (without internalization tracking, timing or launch settings of its
+ * own) runs up to 64 steps per launch; elsewhere runs
  * of more than 16 steps replay a captured CUDA graph of 16 steps (recaptured
  * when the agents, tracking or launch settings change), unless per-step timing
  * is on or the caller is capturing the solve's stream itself; the results are
@@ -498,10 +498,11 @@ void* bfvm_batch_stream(bfvm_batch* batch);
 /* Schedule of a step.  mode 0: one fused persistent launch per step (tiles
  * of every member and sweep from one ordered work list, per-member
  * dependency counters); mode 1: three launches per step (x, y, z), each over
- * the tiles of every member; mode 2: mode 1 for the members under the direct
- * threshold, the others stepped one after another with their own kernels
- * (the tensor-memory sweeps of bfvm_step), all on the batch stream and in
- * its graph.  yz_chunk: rows per TMA box in the y/z sweeps; order (mode 0):
+ * the tiles of every member; mode 2: the members that bfvm_step would run with
+ * several steps per launch side by side in one launch, each on SMs of its own;
+ * of the others, mode 1 for those under the direct threshold, the rest stepped
+ * one after another with their own kernels (the tensor-memory sweeps of
+ * bfvm_step), all on the batch stream and in its graph.  yz_chunk: rows per TMA box in the y/z sweeps; order (mode 0):
  * 0 members as added, 1 largest first; ctas_per_sm (mode 0): 0 = as many as
  * fit; graph_steps: steps per captured CUDA graph.  Every mode gives each
  * member the bits of bfvm_step. */
@@ -509,12 +510,8 @@ int bfvm_batch_set_schedule(bfvm_batch* batch, int mode, int yz_chunk, int order
 int bfvm_batch_get_schedule(bfvm_batch* batch, int* mode, int* yz_chunk, int* order, int* ctas_per_sm,
                             int* graph_steps);
 /* Mode 2: members of at least `values` voxel-substrate values (nx*ny*nz*S,
- * default 2097152 = 128^3 x 1) are stepped with their own kernels.
- * Measured on B200: a mix of 256^3 and 200^3 solves (4 substrates) with 40
- * small ones steps in 1.23 ms under mode 2 against 2.05 ms under mode 1
- * (FP64); the serving workload's FP32 server runs at 7.6e10 against 6.8e10
- * updates/s; 256 uneven solves of edges 24-128 stay faster under mode 1,
- * where the batched sweeps keep the GPU full across members. */
+ * default 2097152 = 128^3 x 1) that do not run side by side with others are
+ * stepped with their own kernels. */
 int bfvm_batch_set_direct_threshold(bfvm_batch* batch, long long values);
 int bfvm_batch_get_direct_threshold(bfvm_batch* batch, long long* values);
 /* Time trial_steps fused steps under each candidate schedule, keep the

@@ -33,11 +33,15 @@ struct bfvm_batch {
   std::vector<unsigned char> h_envs;
   // schedule
   int mode = 0;         // 0: one fused persistent launch per step; 1: three launches (x, y, z) per step;
-                        // 2: as 1 for the members under direct_min values, the others stepped with
-                        // their own kernels (enqueue_step_on) on the batch stream
+                        // 2: the members that bfvm_resident.cu takes side by side in one launch; of the
+                        // others, as 1 those under direct_min values, the rest with their own kernels
+                        // (enqueue_step_on) on the batch stream
   long long direct_min = 2097152;  // mode 2: N*S (voxel-substrate values) from which a member steps directly
   std::vector<bfvm_ctx*> direct;  // mode 2: the members stepped directly (set with the tables)
-  int direct_launches = 0;        // their kernels per step
+  std::vector<bfvm_ctx*> resident;  // mode 2: the members that run side by side in one launch, of either kind
+  bool batched = false;             // there are members under direct_min
+  int direct_launches = 0;        // the kernels per step of the members from direct_min on
+  int resident_launches = 0;      // those of them that stand for stages of the one launch
   // mode 2: the direct members run on up to kSideStreams side streams, forked
   // from the batch stream and joined back around each run of steps, so that
   // the members' own persistent kernels share the GPU; direct_lane[i] is the
@@ -115,17 +119,28 @@ int build_tables(bfvm_batch* b, bool sources) {
   const int n = static_cast<int>(b->members.size());
   int rc = ensure_capacity(b, std::max(n, 1));
   if (rc != BFVM_OK) return rc;
-  // mode 2: the large members step with their own kernels, outside the tables
+  // mode 2: the members that run side by side in one launch and the large ones,
+  // which step with their own kernels, lie outside the tables
   std::vector<int> idx;
   b->direct.clear();
+  b->resident.clear();
+  b->batched = false;
   b->direct_launches = 0;
+  b->resident_launches = 0;
   for (int q = 0; q < n; ++q) {
     bfvm_ctx* c = b->members[q];
-    if (b->mode == 2 && 1LL * c->nx * c->ny * c->nz * c->S >= b->direct_min) {
-      b->direct.push_back(c);
-      b->direct_launches += 3 + ((sources && c->n_agents > 0 && !c->cfg.fuse_sources) ? 1 : 0);
-    } else {
+    const bool direct = b->mode == 2 && 1LL * c->nx * c->ny * c->nz * c->S >= b->direct_min;
+    const bool resident = b->mode == 2 && resident_member<T>(c, sources);
+    if (resident) b->resident.push_back(c);
+    if (resident && !direct) b->batched = true;
+    if (direct) {
+      if (!resident) b->direct.push_back(c);
+      const int launches = 3 + ((sources && c->n_agents > 0 && !c->cfg.fuse_sources) ? 1 : 0);
+      b->direct_launches += launches;
+      if (resident) b->resident_launches += launches;
+    } else if (!resident) {
       idx.push_back(q);
+      b->batched = true;
     }
   }
   // the direct members' side streams: the largest member first onto the
@@ -269,6 +284,9 @@ cudaError_t enqueue_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
       for (int k = 0; k < K; ++k)
         if ((e = cudaStreamWaitEvent(b->side[k], b->fork_ev, 0)) != cudaSuccess) return e;
     }
+    if (e == cudaSuccess && !b->resident.empty())
+      e = run_resident_members<T>(b->resident.data(), static_cast<int>(b->resident.size()), b->built_sources, nsteps,
+                                  b->stream);
     for (int s = 0; s < nsteps && e == cudaSuccess; ++s)
       e = launch_batch_sweeps<T>(b->d_hdr, static_cast<const BatchEnv<T>*>(b->d_envs), b->d_pre, b->cap, b->items,
                                  b->axis_smem, b->stream);
@@ -291,17 +309,18 @@ cudaError_t enqueue_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
 }
 
 // The batched kernels of one step (the directly stepped members count their
-// own launches as they enqueue them).
+// own launches as they enqueue them).  The launch that runs the resident
+// members' steps counts as the stages it stands for.
 int kernels_per_step(const bfvm_batch* b) {
   if (b->mode == 0) return 1;
-  return (b->items[0] > 0) + (b->items[1] > 0) + (b->items[2] > 0);
+  return b->mode == 1 || b->batched ? 3 : 0;
 }
 
 template <typename T>
-int launch_one(bfvm_batch* b, int stall_env = -1) {
-  BFVM_CUDA(enqueue_steps<T>(b, 1, stall_env));
-  note_launches(kernels_per_step(b));
-  b->launches += kernels_per_step(b) + b->direct_launches;
+int launch_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
+  BFVM_CUDA(enqueue_steps<T>(b, nsteps, stall_env));
+  note_launches(nsteps * (kernels_per_step(b) + b->resident_launches));
+  b->launches += nsteps * (kernels_per_step(b) + b->direct_launches);
   return BFVM_OK;
 }
 
@@ -375,9 +394,15 @@ int step_impl(bfvm_batch* b, int nsteps, bool sources) {
     const auto it = std::find(b->members.begin(), b->members.end(), b->stall);
     b->stall = nullptr;
     if (it != b->members.end() && b->mode == 0) {
-      if ((rc = launch_one<T>(b, b->env_of[it - b->members.begin()])) != BFVM_OK) return rc;
+      if ((rc = launch_steps<T>(b, 1, b->env_of[it - b->members.begin()])) != BFVM_OK) return rc;
       --left;
     }
+  }
+  if (!b->resident.empty()) {
+    // every member in the one launch: nothing for a graph to replay
+    const int steps = b->resident.size() == b->members.size() ? left : left % std::max(b->graph_steps, 1);
+    if (steps > 0 && (rc = launch_steps<T>(b, steps)) != BFVM_OK) return rc;
+    left -= steps;
   }
   if (b->graph_steps > 1 && left >= b->graph_steps) {
     if (!b->gexec || b->g_steps != b->graph_steps || b->g_smem != b->smem || b->g_grid != b->grid ||
@@ -393,7 +418,7 @@ int step_impl(bfvm_batch* b, int nsteps, bool sources) {
     }
   }
   for (; left > 0; --left)
-    if ((rc = launch_one<T>(b)) != BFVM_OK) return rc;
+    if ((rc = launch_steps<T>(b, 1)) != BFVM_OK) return rc;
   return release_members(b);
 }
 

@@ -210,6 +210,12 @@ struct NodeLines {
 template <typename T>
 int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, int nsteps, cudaStream_t st,
                  bool* launched);
+// Whether a batch's member may run beside others in run_resident_members, and
+// nsteps whole steps of such members on st.
+template <typename T>
+bool resident_member(bfvm_ctx* c, bool sources);
+template <typename T>
+cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sources, int nsteps, cudaStream_t st);
 cudaError_t resident_set_wait_limit(unsigned long long ns);
 
 inline AgentTrack track_params(const bfvm_ctx* c) {

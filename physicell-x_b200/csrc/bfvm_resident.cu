@@ -11,7 +11,9 @@
 // every warp owns 32 lines per sweep, the sweeps of a step follow one another
 // behind a grid-wide barrier, the sources (and a 2-D step's Dirichlet nodes)
 // are applied by the warp whose x lines hold them, and coefficients and code
-// stay on the SMs from the first step to the last.
+// stay on the SMs from the first step to the last.  Where there are more tiles
+// than warps, and for a batch's solves side by side, resident_many_kernel does
+// the same with several tiles per warp.
 //
 // What a step takes, in cycles at 50x50x50x2 FP64 (156 tiles): per sweep a
 // tile's copy in 1,200-1,500 (one memory latency), forward 2,500 (50 values of
@@ -25,9 +27,11 @@
 //   100x100x100x2 FP64 50.8 -> 28.7 (40.6 -> 26.6)  FP32 49.3 -> 26.2 (40.3 -> 23.9)
 //   128x128x128x1 FP64 52.9 -> 28.8 (43.4 -> 27.0)
 //   300x260 2-D x3 FP64 50.7 -> 30.3 (49.4 -> 27.5); with 10,000 agents and a
-//                 rim of nodes 62.1 -> 51.3 (60.7 -> 46.7)
-// It won at every size it takes, up to what an SM holds: eight warps of 248
-// registers, or 227 KB of line buffers and coefficients.
+//                 rim of nodes 62.1 -> 43.7 (60.6 -> 41.2)
+// With one tile per warp it won at every size it takes, up to what an SM holds:
+// eight warps of 248 registers, or 227 KB of line buffers and coefficients.
+// With several, the next tile's lines prefetched to the L2: see resident_wins;
+// 24 uneven FP32 solves of edges 24 to 128 (247 MB) 594 -> 425 us a step.
 #include <algorithm>
 #include <climits>
 #include <type_traits>
@@ -42,7 +46,9 @@ namespace bfvm {
 
 namespace {
 
+constexpr int kResidentMembers = 48;  // solves per launch at most (their parameters are the launch's: 20 of 32 KB)
 constexpr int kResidentWarps = 8;  // warps per CTA at most
+constexpr int kSpreadThreads = 128;  // at least, of a CTA that takes part in the sources ahead of the x sweep
 constexpr size_t kSmemMax = 227 * 1024;
 constexpr int kAgentBytes = 3 * sizeof(double) + sizeof(int);
 constexpr int kResidentSteps = 64;  // steps per launch at most, about a millisecond: other streams' kernels get a turn
@@ -51,12 +57,13 @@ constexpr int kResidentSteps = 64;  // steps per launch at most, about a millise
 // False once a wait has run out (bounded as every device-side wait here).
 struct GridBarrier {
   unsigned long long* count;
+  unsigned ctas;
   unsigned long long target = 0;
   bool ok = true;
   __device__ __forceinline__ bool sync(int* status) {
     __syncthreads();
     if (threadIdx.x == 0) {
-      target += gridDim.x;
+      target += ctas;
       // this CTA's stores (ordered before by the barrier above) with the arrival
       asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(count), "l"(1ull) : "memory");
       unsigned long long t0 = 0;
@@ -92,6 +99,8 @@ struct ResidentPlan {
   // again every step, kept from its start: agents and nodes (x, y) in lists of
   // these lengths
   int agents, nodes[2];
+  int own;     // one warp: the coefficients of its own tiles' substrates only
+  int spread;  // the sources ahead of the x sweep, by every thread of the run
   int warp_bytes;  // (a multiple of 16, as each list is)
 };
 
@@ -182,9 +191,10 @@ __device__ __forceinline__ ResidentLine<T> resident_line(const SweepParams<T>& p
 // One sweep of one 32-line tile by one warp.  An x sweep's `before` changes
 // the tile in shared memory, and in the field, ahead of the sweep (sources and
 // nodes); its `after` does before the rows go out.
-template <typename T, int AXIS, typename Before, typename After>
+template <typename T, int AXIS, typename Meanwhile, typename Before, typename After>
 __device__ __forceinline__ void resident_tile(const SweepParams<T>& p, const ResidentPlan& pl, const double* coef,
-                                              T* buf, const ResidentLine<T>& l, Before before, After after) {
+                                              T* buf, const ResidentLine<T>& l, Meanwhile meanwhile, Before before,
+                                              After after) {
   using DR = typename Coef<T>::DR;
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int R = kRowBatch, kAhead = 4;  // (kUnits: as many values by units)
@@ -196,8 +206,8 @@ __device__ __forceinline__ void resident_tile(const SweepParams<T>& p, const Res
   const int s = l.s;
   const bool act = l.act, on = l.on, fast = p.screen == kScreenFast;
   const double c1 = l.c1, shift = l.shift, x0 = l.x0, x1 = l.x1;
-  const DR* dr = reinterpret_cast<const DR*>(coef + pl.dr_off[AXIS]) + static_cast<size_t>(s) * pl.rows[AXIS];
-  const double* cu = coef + pl.cu_off[AXIS] + static_cast<size_t>(s) * pl.rows[AXIS];
+  const DR* dr = reinterpret_cast<const DR*>(coef + pl.dr_off[AXIS]) + (pl.own ? 0 : static_cast<size_t>(s) * pl.rows[AXIS]);
+  const double* cu = coef + pl.cu_off[AXIS] + (pl.own ? 0 : static_cast<size_t>(s) * pl.rows[AXIS]);
 
   // ---- the tile in: every copy under way at once (one memory latency for
   // the tile, 1,200 cycles), 16 bytes a lane (8 took three times as long for
@@ -229,6 +239,7 @@ __device__ __forceinline__ void resident_tile(const SweepParams<T>& p, const Res
 #pragma unroll 8
     for (int q = r0; q < n; q += rows, at += rows * stride, to += rows * 32) copy_async16(to, at);
   }
+  meanwhile();
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
   if (AXIS == 0) {
@@ -386,7 +397,7 @@ __device__ __forceinline__ void resident_tile(const SweepParams<T>& p, const Res
 // through it.  The first `kept` agents' data lie in shared memory for the run,
 // as do a plane's nodes: 300x260x3 FP64 with 10,000 agents and a rim of nodes,
 // three solves at once, took 26 us a step with both read from memory each time
-// and takes 17.  Agents in a face line of an activated substrate are
+// and takes 15.  Agents in a face line of an activated substrate are
 // left out: the line is pinned before anything reads it (no agents are tracked
 // here).
 struct ResidentAgent {
@@ -424,7 +435,7 @@ __device__ __forceinline__ ResidentAgent resident_agent(const SweepParams<T>& p,
   return a;
 }
 
-template <typename T>
+template <int ROUNDS, typename T>
 __device__ __forceinline__ ResidentAgents<T> resident_agents(const SweepParams<T>& p, int tile, int cap, double* keep) {
   ResidentAgents<T> g{};
   const int rows = p.ny * p.nz, per_s = (rows + 31) / 32, t = threadIdx.x & 31;
@@ -444,12 +455,20 @@ __device__ __forceinline__ ResidentAgents<T> resident_agents(const SweepParams<T
   g.cap = cap;
   g.k = keep;
   g.at = reinterpret_cast<int*>(keep + 3 * cap);
-  for (int e = t; e < g.kept; e += 32) {
-    const ResidentAgent a = resident_agent(p, g, g.a0 + e);
-    g.k[e] = a.k1;
-    g.k[e + cap] = a.k2;
-    g.k[e + 2 * cap] = a.k3;
-    g.at[e] = a.at;
+  constexpr int kRounds = ROUNDS;  // read together: one memory latency
+  for (int e0 = t; e0 < g.kept; e0 += 32 * kRounds) {
+    ResidentAgent a[kRounds];
+#pragma unroll
+    for (int u = 0; u < kRounds; ++u) a[u] = resident_agent(p, g, g.a0 + min(e0 + 32 * u, g.kept - 1));
+#pragma unroll
+    for (int u = 0; u < kRounds; ++u) {
+      const int e = e0 + 32 * u;
+      if (e >= g.kept) break;
+      g.k[e] = a[u].k1;
+      g.k[e + cap] = a[u].k2;
+      g.k[e + 2 * cap] = a[u].k3;
+      g.at[e] = a[u].at;
+    }
   }
   return g;
 }
@@ -482,6 +501,28 @@ __device__ __forceinline__ void resident_sources(const SweepParams<T>& p, const 
     tile[static_cast<size_t>(row) * p.nxp + i] = x;
   }
   __syncwarp();
+}
+
+// The sources by all of the run's threads, thread `id` of `threads`, ahead of
+// the x sweep and a barrier: where many agents lie in a tile.
+template <typename T>
+__device__ __forceinline__ void resident_spread(const SweepParams<T>& p, long long id, long long threads) {
+  const int rows = p.ny * p.nz, n = __ldg(p.line_off + rows);
+  for (long long e = id; e < static_cast<long long>(n) * p.S; e += threads) {
+    const int s = static_cast<int>(e / n), q = static_cast<int>(e - static_cast<long long>(s) * n);
+    const unsigned key = __ldg(p.a_key + q), before = __ldg(p.a_key + max(q - 1, 0));
+    const size_t sn = static_cast<size_t>(s) * p.n_sorted;
+    const double k1 = __ldg(p.ac1 + sn + q), k2 = __ldg(p.ac2 + sn + q), k3 = __ldg(p.ae2 + sn + q);
+    if (q > 0 && before == key) continue;
+    const int row = static_cast<int>(key / p.nx), i = static_cast<int>(key - static_cast<unsigned>(row) * p.nx);
+    const int k = row / p.ny, j = row - k * p.ny;
+    if (p.active[s] != 0 && (j == 0 || j == p.ny - 1 || k == 0 || k == p.nz - 1)) continue;
+    T* const rho = p.f + (static_cast<size_t>(s) * rows + row) * p.nxp + i;
+    T x = __ldcg(rho);
+    apply_run<T>(&x, q, key, k1, k2, k3, n, p.a_key, p.ac1 + sn, p.ac2 + sn, p.ae2 + sn,
+                 sizeof(T) == 4 ? p.off[s] : 0.0, s, p.track);
+    *rho = x;
+  }
 }
 
 // The y and z face lines of activated substrates take their face's values
@@ -597,26 +638,81 @@ __device__ __forceinline__ void resident_pin(const SweepParams<T>& p, const Resi
   __syncwarp();
 }
 
+// A tile's 128-byte lines (a row's start on them) on their way to the L2.
+template <typename T, int AXIS>
+__device__ __forceinline__ void resident_prefetch(const SweepParams<T>& p, int tile, int tiles) {
+  if (tile >= tiles) return;
+  const int t = threadIdx.x & 31;
+  constexpr int kLine = 128 / sizeof(T);
+  const T* at;
+  size_t step;
+  int count;
+  if (AXIS == 0) {
+    const int rows = p.ny * p.nz, per_s = (rows + 31) / 32, s = tile / per_s, r0 = (tile - s * per_s) * 32;
+    at = p.f + (static_cast<size_t>(s) * rows + r0) * p.nxp + t * kLine;
+    step = 32 * kLine;
+    count = min(32, rows - r0) * (p.nxp / kLine);
+  } else {
+    constexpr int kLines = 32 / kLine;  // per row
+    const int nm = AXIS == 1 ? p.nz : p.ny, n = AXIS == 1 ? p.ny : p.nz;
+    const int xt = (p.nx + 31) / 32, per_s = xt * nm, s = tile / per_s, q = tile - s * per_s, m = q / xt;
+    const size_t stride = resident_stride<T, AXIS>(p);
+    at = p.f + (AXIS == 1 ? (static_cast<size_t>(s) * p.nz + m) * p.ny : static_cast<size_t>(s) * p.nz * p.ny + m) * p.nxp +
+         (q - m * xt) * 32 + t / kLines * stride + t % kLines * kLine;
+    step = 32 / kLines * stride;
+    count = n * kLines;
+  }
+  for (int q = t; q < count; q += 32, at += step) asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+}
+
+// A run's coefficients to shared memory, every copy under way at once (a plane's
+// CTA has one warp: with a loop of loads a call of one step of 300x260x3 took
+// 67 us, its steps 39).
 template <typename T>
-__global__ void __launch_bounds__(32 * kResidentWarps, 1)
-    resident_kernel(const SweepParams<T> p, const ResidentPlan pl, const NodeLines nd, unsigned long long* barrier) {
-  using DR = typename Coef<T>::DR;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* const coef = reinterpret_cast<double*>(smem_raw + static_cast<size_t>(pl.warps) * pl.warp_bytes);
+__device__ __forceinline__ double* resident_coefs(const SweepParams<T>& p, const ResidentPlan& pl, unsigned char* smem,
+                                                  int sx, int sy, int sz) {
+  constexpr int kDR = sizeof(typename Coef<T>::DR) / sizeof(double);
+  double* const coef = reinterpret_cast<double*>(smem + static_cast<size_t>(pl.warps) * pl.warp_bytes);
   const AxisCoefs<T>* axes[3] = {&p.ax, &p.ay, &p.az};
   const int naxes = pl.two_d ? 2 : 3;
   for (int a = 0; a < naxes; ++a) {
-    const int rows = pl.rows[a], npad = axes[a]->npad;
-    DR* dr = reinterpret_cast<DR*>(coef + pl.dr_off[a]);
-    for (int q = threadIdx.x; q < rows * p.S; q += blockDim.x) {
-      const int s = q / rows, r = q - s * rows;
-      dr[q] = __ldg(axes[a]->dr + static_cast<size_t>(s) * npad + r);
-      coef[pl.cu_off[a] + q] = __ldg(axes[a]->cu + static_cast<size_t>(s) * npad + r);
+    const int rows = pl.rows[a];  // (even, and the padded rows too: 16 bytes are whole)
+    const int s0 = pl.own ? (a == 0 ? sx : (a == 1 ? sy : sz)) : 0, ns = pl.own ? 1 : p.S;
+    for (int q0 = 0; q0 < ns; ++q0) {
+      const int s = s0 + q0;
+      const double* dr = reinterpret_cast<const double*>(axes[a]->dr + static_cast<size_t>(s) * axes[a]->npad);
+      const double* cu = axes[a]->cu + static_cast<size_t>(s) * axes[a]->npad;
+      double* const to = coef + pl.dr_off[a] + q0 * rows * kDR;
+      for (int q = 2 * threadIdx.x; q < rows * kDR; q += 2 * blockDim.x) copy_async16(to + q, dr + q);
+      for (int q = 2 * threadIdx.x; q < rows; q += 2 * blockDim.x)
+        copy_async16(coef + pl.cu_off[a] + q0 * rows + q, cu + q);
     }
   }
+  return coef;  // (there once the caller has waited for its copies)
+}
+
+// The last of the run's CTAs leaves the counters at zero for the next run.
+__device__ __forceinline__ void resident_leave(unsigned long long* barrier, int ctas) {
   __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(barrier + 1, 1ull) == ctas - 1) {
+      barrier[0] = 0;
+      barrier[1] = 0;
+    }
+  }
+}
+
+// One tile per warp and axis: all that does not change from step to step is
+// set up once.
+template <typename T>
+__global__ void __launch_bounds__(32 * kResidentWarps, 1)
+    resident_kernel(const SweepParams<T> p, const ResidentPlan pl, const NodeLines nd, unsigned long long* barrier) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5;
-  const int w0 = blockIdx.x + gridDim.x * warp, nw = gridDim.x * pl.warps;  // neighbouring tiles on different SMs
+  // Neighbouring tiles on different SMs.  (Warps past the plan's, there for the
+  // sources, find no tile.)
+  const int w0 = blockIdx.x + gridDim.x * warp, nw = gridDim.x * (blockDim.x >> 5);
   unsigned char* keep = smem_raw + static_cast<size_t>(warp) * pl.warp_bytes;
   T* const buf = reinterpret_cast<T*>(keep);
   const int pitch = resident_pitch<T>(p.nx);
@@ -624,7 +720,13 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   const ResidentLine<T> lx = resident_line<T, 0>(p, w0), ly = resident_line<T, 1>(p, w0);
   ResidentLine<T> lz{};
   if (!pl.two_d) lz = resident_line<T, 2>(p, w0);
-  const ResidentAgents<T> ag = resident_agents(p, w0, pl.agents, reinterpret_cast<double*>(keep));
+  // (own: warp 0's tiles are the CTA's)
+  const int cta = blockIdx.x, xt = (p.nx + 31) / 32;
+  const double* const coef =
+      resident_coefs(p, pl, smem_raw, min(cta / ((p.ny * p.nz + 31) / 32), p.S - 1), min(cta / (xt * p.nz), p.S - 1),
+                     min(cta / (xt * p.ny), p.S - 1));
+  ResidentAgents<T> ag{};
+  if (!pl.spread) ag = resident_agents<4>(p, w0, pl.agents, reinterpret_cast<double*>(keep));
   keep += static_cast<size_t>(pl.agents) * kAgentBytes;
   const ResidentNodes<T> xn = resident_nodes(p, nd, 0, w0, pl.nodes[0], keep);
   keep += static_cast<size_t>(pl.nodes[0]) * (sizeof(T) + sizeof(int));
@@ -633,11 +735,17 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   __syncwarp();
   ResidentFace<T> face{};
   if (w0 < pl.face_rows) face = resident_face(p, w0);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
   const auto none = [] {};
-  GridBarrier bar{barrier};
+  GridBarrier bar{barrier, gridDim.x};
   for (int step = 0; step < pl.nsteps; ++step) {
+    if (pl.spread) {
+      resident_spread(p, w0 * 32ll + (threadIdx.x & 31), nw * 32ll);
+      if (!bar.sync(p.status)) break;
+    }
     resident_tile<T, 0>(
-        p, pl, coef, buf, lx,
+        p, pl, coef, buf, lx, none,
         [&] {
           if (ag.a1 > ag.a0) resident_sources(p, ag, buf, pitch, lx.tile);
           if (xn.n > 0) resident_pin(p, xn, true, buf, pitch, l0);
@@ -648,23 +756,248 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
     resident_face_store(face, p.nx);
     for (int q = w0 + nw; q < pl.face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
     if (!bar.sync(p.status)) break;
-    resident_tile<T, 1>(p, pl, coef, buf, ly, none, none);
+    resident_tile<T, 1>(p, pl, coef, buf, ly, none, none, none);
     if (yn.n > 0) resident_pin<T>(p, yn, true, nullptr, 0, 0);
     if (!pl.two_d) {
       if (!bar.sync(p.status)) break;
-      resident_tile<T, 2>(p, pl, coef, buf, lz, none, none);
+      resident_tile<T, 2>(p, pl, coef, buf, lz, none, none, none);
     }
     if (step + 1 < pl.nsteps && !bar.sync(p.status)) break;
   }
-  // the launch's last CTA leaves the counters at zero for the next one
+  resident_leave(barrier, gridDim.x);
+}
+
+// Several tiles per warp and axis, and several solves side by side: each has
+// CTAs cta0 .. cta0 + ctas - 1 and a barrier of its own, so a batch's solves
+// go through their steps independently.
+template <typename T>
+struct ResidentSolve {
+  SweepParams<T> p;
+  ResidentPlan pl;
+  int cta0, ctas;
+  unsigned long long* barrier;
+};
+
+template <typename T, int N>
+struct ResidentBatch {
+  int n, nsteps;
+  ResidentSolve<T> solve[N];
+};
+
+// Warps per CTA at most: FP32's eight and sixteen were no faster (24 solves
+// side by side: 420 us a step with any; 100 smaller ones 642 with 8 and 12, 725
+// with 16), FP64's twelve neither, as shared memory holds fewer from 100 values
+// a line on.
+template <typename T>
+constexpr int kManyWarps = sizeof(T) == 4 ? 12 : 8;
+
+template <typename T, int N>
+__global__ void __launch_bounds__(32 * kManyWarps<T>, 1) resident_many_kernel(const __grid_constant__ ResidentBatch<T, N> b) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  int m = 0;
+  if constexpr (N > 1) {
+    while (m + 1 < b.n && static_cast<int>(blockIdx.x) >= b.solve[m + 1].cta0) ++m;
+  }
+  const SweepParams<T>& p = b.solve[m].p;
+  const ResidentPlan& pl = b.solve[m].pl;
+  const int ctas = b.solve[m].ctas;
+  const double* const coef = resident_coefs(p, pl, smem_raw, 0, 0, 0);
+  const int warp = threadIdx.x >> 5;
+  const int nw = ctas * pl.warps;
+  // (a warp past the solve's takes part in the barriers only)
+  const int w0 = warp < pl.warps ? static_cast<int>(blockIdx.x) - b.solve[m].cta0 + ctas * warp : INT_MAX / 2;
+  unsigned char* const keep = smem_raw + static_cast<size_t>(warp) * pl.warp_bytes;
+  T* const buf = reinterpret_cast<T*>(keep);
+  double* const agents = reinterpret_cast<double*>(keep + static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T));
+  const int pitch = resident_pitch<T>(p.nx);
+  const int xt = (p.nx + 31) / 32;
+  const int ntx = (p.ny * p.nz + 31) / 32 * p.S, nty = xt * p.nz * p.S, ntz = xt * p.ny * p.S;
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(barrier + 1, 1ull) == gridDim.x - 1) {
-      barrier[0] = 0;
-      barrier[1] = 0;
+  const auto none = [] {};
+  GridBarrier bar{b.solve[m].barrier, static_cast<unsigned>(ctas)};
+  for (int step = 0; step < b.nsteps; ++step) {
+    for (int q = w0; q < pl.face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
+    if (pl.spread) {
+      resident_spread(p, static_cast<long long>(blockIdx.x - b.solve[m].cta0) * blockDim.x + threadIdx.x,
+                      static_cast<long long>(ctas) * blockDim.x);
+      if (!bar.sync(p.status)) break;
+    }
+    for (int tile = w0; tile < ntx; tile += nw) {
+      ResidentAgents<T> ag{};
+      const ResidentLine<T> l = resident_line<T, 0>(p, tile);
+      resident_tile<T, 0>(
+          p, pl, coef, buf, l, [&] {
+            resident_prefetch<T, 0>(p, tile + nw, ntx);
+            if (!pl.spread) ag = resident_agents<1>(p, tile, pl.agents, agents);
+          },
+          [&] {
+            if (ag.a1 > ag.a0) resident_sources(p, ag, buf, pitch, l.tile);
+          },
+          none);
+    }
+    if (!bar.sync(p.status)) break;
+    for (int tile = w0; tile < nty; tile += nw)
+      resident_tile<T, 1>(p, pl, coef, buf, resident_line<T, 1>(p, tile),
+                          [&] { resident_prefetch<T, 1>(p, tile + nw, nty); }, none, none);
+    if (!bar.sync(p.status)) break;
+    for (int tile = w0; tile < ntz; tile += nw)
+      resident_tile<T, 2>(p, pl, coef, buf, resident_line<T, 2>(p, tile),
+                          [&] { resident_prefetch<T, 2>(p, tile + nw, ntz); }, none, none);
+    if (step + 1 < b.nsteps && !bar.sync(p.status)) break;
+  }
+  resident_leave(b.solve[m].barrier, ctas);
+}
+
+// Whether the sources go ahead of the x sweep, spread over `threads` threads.
+// x tiles take them 32 at a time, about 1,000 cycles (an exact division, then
+// the runs of stacked agents), `rounds` tiles one after another; the spread
+// phase takes a barrier and about 2,000 cycles for each agent of a thread.
+// us per step, FP64, 10 steps, in the tiles -> spread: a plane of 537x74x3 with
+// 2,000 agents (20 rounds) 41 -> 33, with 8,000 (83) 100 -> 34; 200x200x200x1
+// with 1.6 million (3 x 40 rounds, 42 spread) 250 -> 182; but 64x64x64x8 FP32
+// with 52,000 (13 rounds, 11 spread) 25 -> 36.
+template <typename T>
+bool resident_spreads(const bfvm_ctx* c, const SweepParams<T>& p, long long rounds, long long threads) {
+  if (p.line_off == nullptr) return false;
+  const long long tiles = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
+  const long long in_tiles = rounds * ((c->n_agents / tiles + 31) / 32);
+  return in_tiles > 8 + 2 * ((static_cast<long long>(c->n_agents) * c->S + threads - 1) / threads);
+}
+
+// Shapes and shared memory of a solve's run, with one tile per warp (many
+// false) or several; false where it does not fit.
+template <typename T>
+bool resident_plan(const bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, bool many, int sms,
+                   ResidentPlan* plan, long long* tiles, size_t* smem) {
+  const SweepConfig& g = c->cfg;
+  if (c->timing || (p.line_off != nullptr && c->track) || c->sub_streams != 1 || g.persistent != 1 || g.tmem != 1 ||
+      g.x_lines != 32 || g.yz_tile != 32)
+    return false;
+  const int n[3] = {c->nx, c->ny, c->nz}, S = c->S;
+  const int naxes = two_d ? 2 : 3;
+  ResidentPlan pl{};
+  pl.two_d = two_d ? 1 : 0;
+  if (!two_d) {
+    int on = 0;
+    for (int s = 0; s < S; ++s) on += c->active[s] ? 1 : 0;
+    const int zrows = (c->nz > 1 ? 2 : 1) * c->ny, yrows = (c->ny > 1 ? 2 : 1) * (c->nz > 2 ? c->nz - 2 : 0);
+    pl.face_rows = on * (zrows + yrows);
+  }
+  const long long xt = (c->nx + 31) / 32, xrows = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
+  tiles[0] = xrows * S;
+  tiles[1] = xt * c->nz * S;
+  tiles[2] = two_d ? 0 : xt * c->ny * S;
+  const long long most = std::max(tiles[0], std::max(tiles[1], tiles[2]));
+  if (most >= INT_MAX / 2) return false;
+  const long long ctas = std::min<long long>(most, sms), per_cta = (most + ctas - 1) / ctas;
+  pl.own = !many && per_cta == 1 ? 1 : 0;
+  const size_t sets = pl.own ? 1 : S;
+  size_t doubles = 0;
+  const int drd = sizeof(typename Coef<T>::DR) / 8;
+  for (int a = 0; a < naxes; ++a) {
+    pl.rows[a] = (n[a] + kRowBatch - 1) / kRowBatch * kRowBatch;
+    pl.line = std::max(pl.line, n[a]);
+    pl.dr_off[a] = static_cast<int>(doubles);
+    doubles += static_cast<size_t>(drd) * pl.rows[a] * sets;
+    pl.cu_off[a] = static_cast<int>(doubles);
+    doubles += static_cast<size_t>(pl.rows[a]) * sets;
+    if (doubles * sizeof(double) > kSmemMax) return false;
+  }
+  const size_t coefs = doubles * sizeof(double);
+  size_t each = static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T);
+  for (int a = 0; a < 2 && nodes.n > 0; ++a) {
+    pl.nodes[a] = (nodes.most[a] + 3) / 4 * 4;
+    each += static_cast<size_t>(pl.nodes[a]) * (sizeof(T) + sizeof(int));
+  }
+  if (many) {
+    pl.agents = p.line_off != nullptr ? 32 : 0;
+    each += static_cast<size_t>(pl.agents) * kAgentBytes;
+    pl.warps = static_cast<int>(std::min<size_t>(kManyWarps<T>, (kSmemMax - coefs) / each));
+    if (pl.warps < 1) return false;
+  } else {
+    if (per_cta > kResidentWarps || per_cta * each + coefs > kSmemMax) return false;
+    pl.warps = static_cast<int>(per_cta);
+    pl.spread = resident_spreads(c, p, 1, static_cast<long long>(sms) * kSpreadThreads) ? 1 : 0;
+    if (p.line_off != nullptr && !pl.spread) {  // room for a tile of twice the average, or what there is
+      const long long fit = static_cast<long long>((kSmemMax - coefs) / pl.warps - each) / kAgentBytes;
+      pl.agents = static_cast<int>(std::min<long long>(fit, 2 * (c->n_agents / xrows) + 32) / 4 * 4);
+      each += static_cast<size_t>(pl.agents) * kAgentBytes;
     }
   }
+  pl.warp_bytes = static_cast<int>(each);
+  *plan = pl;
+  *smem = pl.warps * each + coefs;
+  return true;
+}
+
+template <typename T, int N>
+cudaError_t launch_many(ResidentBatch<T, N>& b, int grid, size_t smem, int warps, int nsteps, cudaStream_t st) {
+  int blocks = 0;
+  cudaError_t e = persistent_grid(resident_many_kernel<T, N>, smem, grid, &blocks, 32 * warps);
+  if (e != cudaSuccess) return e;
+  if (blocks < grid) return cudaErrorLaunchOutOfResources;
+  for (int done = 0; done < nsteps && e == cudaSuccess; done += b.nsteps) {
+    b.nsteps = std::min(kResidentSteps, nsteps - done);
+    void* args[] = {&b};
+    e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(resident_many_kernel<T, N>), dim3(grid),
+                                    dim3(32 * warps), args, smem, st);
+  }
+  return e;
+}
+
+// Whether a solve with several tiles per warp is faster this way than with a
+// launch per stage.  us per step, 10 steps a call, a launch per stage -> this:
+//   FP64 100x100x100x3 71.9 -> 43.5   128x128x128x4 114 -> 78   200x200x200x1 136 -> 104
+//        100x100x100x10 (80 MB) 130 -> 126, 64 steps 119 -> 123; 160x160x160x3
+//        (98 MB) 152 -> 152, 140 -> 150; 200x200x200x4 (256 MB) 336 -> 428
+//   FP32 100x100x100x3 54.6 -> 31.2   128x128x128x8 132 -> 89   200x200x200x2 169 -> 112
+//        300x300x300x1 (108 MB) 264 -> 242, 200x200x200x4 (128 MB) 254 -> 236,
+//        300x300x300x2 (216 MB) 409 -> 458
+// Its warps hide an L2 latency, not DRAM's: the field has to stay in the L2, in
+// FP64, with half the warps, well inside it.  And lines that leave room for
+// fewer than three warps an SM are a serial chain with nothing beside it: FP64
+// 256x128x128 (three) 98 -> 70, 300x100x100 (two) 73 -> 75, 400x64x64x2 (two)
+// 81 -> 120.
+template <typename T>
+bool resident_wins(const bfvm_ctx* c, const ResidentPlan& pl) {
+  int l2 = 0;
+  if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c->device) != cudaSuccess) return false;
+  const double bytes = static_cast<double>(sizeof(T)) * c->nx * c->ny * c->nz * c->S;
+  return pl.warps >= 3 && bytes <= (sizeof(T) == 4 ? 1.0 : 0.55) * l2;
+}
+
+// And for a solve that has the GPU to itself or shares it with others on
+// streams of their own, which a launch per stage leaves more room for.  us per
+// call, FP32 unless stated, a launch per stage -> this, alone and three at once:
+//   64x64x64x8 (seven warps an SM): 1 step 37 -> 28 and 19 -> 24, 4 steps 143 ->
+//     78 and 71 -> 75, 10 steps 354 -> 178 and 177 -> 174; 50x50x50x2 FP64 (two
+//     warps) 1 step 32 -> 22 and 22 -> 10
+//   ten steps of 58x25x184x2 (five warps, their lanes 0.25 busy: 736 y tiles, 100
+//     z tiles) 391 -> 186 and 163 -> 182; 120x30x30x6 FP64 (0.46) 370 -> 175 and
+//     161 -> 172, 33x47x61x7 FP64 (0.50) 339 -> 173 and 170 -> 169; several tiles
+//     per warp: 58x25x184x4 (0.46) 411 -> 222 and 182 -> 218, 100x100x100x3 FP64
+//     (0.63) 702 -> 419 and 402 -> 416, 200x200x200x1 FP64 (0.70) 1357 -> 1027
+//     and 1111 -> 1034, 128x128x128x4 (0.99) 771 -> 511 and 547 -> 511
+//   with agents in 1 voxel of 17: 100x100x100x3 FP64 702 -> 499 and 437 -> 502,
+//     120x30x30x6 370 -> 205 and 163 -> 203: a tile takes them 32 at a time, a
+//     launch of its own with all threads
+// so more than four warps an SM come with four steps and more, agents in less
+// than 1 voxel of 32, and lanes that are busy.
+template <typename T>
+bool resident_shares(const bfvm_ctx* c, const SweepParams<T>& p, const long long* tiles, long long warps, int nsteps,
+                     double busy) {
+  const long long voxels = static_cast<long long>(c->nx) * c->ny * c->nz;
+  if (nsteps < 4 || (p.line_off != nullptr && 32ll * c->n_agents > voxels)) return false;
+  const long long n[3] = {c->nx, c->ny, c->nz};
+  double slots = 0;  // values that the warps' lanes could take meanwhile
+  for (int a = 0; a < 3; ++a) slots += static_cast<double>((tiles[a] + warps - 1) / warps * warps) * 32 * n[a];
+  return 3.0 * voxels * c->S >= busy * slots;
+}
+
+int sm_count(int device, int* sms) {
+  BFVM_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, device));
+  return BFVM_OK;
 }
 
 }  // namespace
@@ -673,71 +1006,131 @@ template <typename T>
 int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, int nsteps, cudaStream_t st,
                  bool* launched) {
   *launched = false;
-  const SweepConfig& g = c->cfg;
-  if (nsteps < 1 || c->timing || (p.line_off != nullptr && c->track) || c->sub_streams != 1 || g.persistent != 1 ||
-      g.tmem != 1 || g.x_lines != 32 || g.yz_tile != 32)
-    return BFVM_OK;
-  const int n[3] = {c->nx, c->ny, c->nz}, S = c->S;
-  const int naxes = two_d ? 2 : 3;
-  ResidentPlan pl{};
-  pl.two_d = two_d ? 1 : 0;
-  size_t doubles = 0;
-  const int drd = sizeof(typename Coef<T>::DR) / 8;
-  for (int a = 0; a < naxes; ++a) {
-    pl.rows[a] = (n[a] + kRowBatch - 1) / kRowBatch * kRowBatch;
-    pl.line = std::max(pl.line, n[a]);
-    pl.dr_off[a] = static_cast<int>(doubles);
-    doubles += static_cast<size_t>(drd) * pl.rows[a] * S;
-    pl.cu_off[a] = static_cast<int>(doubles);
-    doubles += static_cast<size_t>(pl.rows[a]) * S;
-    if (doubles * sizeof(double) > kSmemMax) return BFVM_OK;
-  }
-  if (!two_d) {
-    int on = 0;
-    for (int s = 0; s < S; ++s) on += c->active[s] ? 1 : 0;
-    const int zrows = (c->nz > 1 ? 2 : 1) * c->ny, yrows = (c->ny > 1 ? 2 : 1) * (c->nz > 2 ? c->nz - 2 : 0);
-    pl.face_rows = on * (zrows + yrows);
-  }
-  const long long xt = (c->nx + 31) / 32;
-  long long tiles = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
-  tiles = std::max(tiles, xt * c->nz);
-  if (!two_d) tiles = std::max(tiles, xt * c->ny);
-  tiles *= S;
+  if (nsteps < 1) return BFVM_OK;
   int sms = 0;
-  BFVM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-  const int grid = static_cast<int>(std::min<long long>(tiles, sms));
-  const long long warps = (tiles + grid - 1) / grid;
-  if (warps > kResidentWarps) return BFVM_OK;
-  pl.warps = static_cast<int>(warps);
-  const size_t coefs = doubles * sizeof(double);
-  size_t each = static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T);
-  for (int a = 0; a < 2 && nodes.n > 0; ++a) {
-    pl.nodes[a] = (nodes.most[a] + 3) / 4 * 4;
-    each += static_cast<size_t>(pl.nodes[a]) * (sizeof(T) + sizeof(int));
-  }
-  if (warps * each + coefs > kSmemMax) return BFVM_OK;
-  if (p.line_off != nullptr) {  // room for the agents of a tile with twice the average, or what there is
-    const long long rows = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
-    const long long fit = static_cast<long long>((kSmemMax - coefs) / warps - each) / kAgentBytes;
-    pl.agents = static_cast<int>(std::min<long long>(fit, 2 * (c->n_agents / rows) + 32) / 4 * 4);
-    each += static_cast<size_t>(pl.agents) * kAgentBytes;
-  }
-  pl.warp_bytes = static_cast<int>(each);
-  const size_t smem = warps * each + coefs;
-  int blocks = 0;
-  BFVM_CUDA(persistent_grid(resident_kernel<T>, smem, grid, &blocks, 32 * pl.warps));
-  if (blocks < grid) return BFVM_OK;
+  const int rc = sm_count(c->device, &sms);
+  if (rc != BFVM_OK) return rc;
+  ResidentPlan pl;
+  long long tiles[3];
+  size_t smem = 0;
   unsigned long long* barrier = c->d_tile_counter + 4;
-  for (int done = 0; done < nsteps; done += pl.nsteps) {
-    pl.nsteps = std::min(kResidentSteps, nsteps - done);
-    void* args[] = {const_cast<SweepParams<T>*>(&p), &pl, const_cast<NodeLines*>(&nodes), &barrier};
-    BFVM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(resident_kernel<T>), dim3(grid),
-                                          dim3(32 * pl.warps), args, smem, st));
+  if (resident_plan(c, p, nodes, two_d, false, sms, &pl, tiles, &smem)) {
+    int grid = static_cast<int>(std::min<long long>(std::max(tiles[0], std::max(tiles[1], tiles[2])), sms));
+    if (pl.warps > 4 && !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.45))
+      return BFVM_OK;
+    int threads = 32 * pl.warps;
+    if (pl.spread) {
+      // Eight agents a thread, and two CTAs to an SM where their lines allow it:
+      // a small grid leaves SMs to others' work (600x500x4 FP32 with 18,000
+      // agents, 10 steps, three solves at once: 469 us a call on all SMs).
+      const long long ctas = (static_cast<long long>(c->n_agents) * c->S + 8 * kSpreadThreads - 1) / (8 * kSpreadThreads);
+      grid = static_cast<int>(std::max<long long>(grid, std::min<long long>(ctas, sms)));
+      threads = std::max(threads, kSpreadThreads);
+    }
+    int blocks = 0;
+    BFVM_CUDA(persistent_grid(resident_kernel<T>, smem, grid, &blocks, threads));
+    if (blocks < grid) return BFVM_OK;
+    for (int done = 0; done < nsteps; done += pl.nsteps) {
+      pl.nsteps = std::min(kResidentSteps, nsteps - done);
+      void* args[] = {const_cast<SweepParams<T>*>(&p), &pl, const_cast<NodeLines*>(&nodes), &barrier};
+      BFVM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(resident_kernel<T>), dim3(grid),
+                                            dim3(threads), args, smem, st));
+    }
+    *launched = true;
+    return BFVM_OK;
   }
-  *launched = true;
+  if (!two_d && resident_plan(c, p, nodes, false, true, sms, &pl, tiles, &smem)) {
+    const long long most = std::max(tiles[0], std::max(tiles[1], tiles[2]));
+    const int grid = static_cast<int>(std::min<long long>(most, sms));
+    const long long all = static_cast<long long>(grid) * pl.warps, rounds = (most + all - 1) / all;
+    // no more warps than that many rounds need
+    const int warps = static_cast<int>((most + grid * rounds - 1) / (grid * rounds));
+    if (!resident_wins<T>(c, pl) || !resident_shares(c, p, tiles, static_cast<long long>(grid) * warps, nsteps, 0.65))
+      return BFVM_OK;
+    smem -= static_cast<size_t>(pl.warps - warps) * pl.warp_bytes;
+    pl.warps = warps;
+    const long long all_x = static_cast<long long>(grid) * warps;
+    pl.spread = resident_spreads(c, p, (tiles[0] + all_x - 1) / all_x, 32ll * grid * kManyWarps<T>) ? 1 : 0;
+    ResidentBatch<T, 1> b{};
+    b.n = 1;
+    b.solve[0] = {p, pl, 0, grid, barrier};
+    BFVM_CUDA(launch_many(b, grid, smem, pl.spread ? kManyWarps<T> : warps, nsteps, st));
+    *launched = true;
+  }
   return BFVM_OK;
 }
 
+// ---- a batch's solves ------------------------------------------------------
+
+template <typename T>
+bool resident_member(bfvm_ctx* c, bool sources) {
+  int sms = 0;
+  ResidentPlan pl;
+  long long tiles[3];
+  size_t smem;
+  return sm_count(c->device, &sms) == BFVM_OK &&
+         resident_plan(c, make_params<T>(c, sources), NodeLines{}, false, true, sms, &pl, tiles, &smem) &&
+         resident_wins<T>(c, pl);
+}
+
+template <typename T>
+cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sources, int nsteps, cudaStream_t st) {
+  ResidentBatch<T, kResidentMembers> b{};
+  int sms = 0;
+  if (count == 0 || sm_count(members[0]->device, &sms) != BFVM_OK) return cudaGetLastError();
+  for (int m0 = 0; m0 < count; m0 += b.n) {
+    b.n = std::min(count - m0, std::min(kResidentMembers, sms));
+    long long tiles[kResidentMembers][3];
+    size_t smem = 0;
+    int warps = 0;
+    for (int m = 0; m < b.n; ++m) {
+      bfvm_ctx* c = members[m0 + m];
+      ResidentSolve<T>& s = b.solve[m];
+      size_t need = 0;
+      s.p = make_params<T>(c, sources);
+      if (!resident_plan(c, s.p, NodeLines{}, false, true, sms, &s.pl, tiles[m], &need)) return cudaErrorInvalidValue;
+      s.barrier = c->d_tile_counter + 4;
+      s.ctas = 1;
+      smem = std::max(smem, need);
+      warps = std::max(warps, s.pl.warps);
+    }
+    // The SMs to the solves, one by one to the one that would take longest: a
+    // tile's time goes with its line (cycles measured at 50 to 128 values).
+    auto time = [&](int m) {
+      const bfvm_ctx* c = members[m0 + m];
+      const ResidentSolve<T>& s = b.solve[m];
+      const int n[3] = {c->nx, c->ny, c->nz};
+      const long long w = static_cast<long long>(s.ctas) * s.pl.warps;
+      long long t = 0;
+      for (int a = 0; a < 3; ++a) t += (tiles[m][a] + w - 1) / w * (2000 + 100 * n[a]) + 2500;
+      return t;
+    };
+    long long took[kResidentMembers];
+    for (int m = 0; m < b.n; ++m) took[m] = time(m);
+    int grid = b.n;
+    for (; grid < sms; ++grid) {
+      const int worst = static_cast<int>(std::max_element(took, took + b.n) - took);
+      ++b.solve[worst].ctas;
+      took[worst] = time(worst);
+    }
+    int cta = 0;
+    for (int m = 0; m < b.n; ++m) {
+      b.solve[m].cta0 = cta;
+      const long long w = static_cast<long long>(b.solve[m].ctas) * b.solve[m].pl.warps;
+      b.solve[m].pl.spread =
+          resident_spreads(members[m0 + m], b.solve[m].p, (tiles[m][0] + w - 1) / w, 32ll * warps * b.solve[m].ctas) ? 1 : 0;
+      cta += b.solve[m].ctas;
+    }
+    const cudaError_t e = launch_many(b, grid, smem, warps, nsteps, st);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
+template bool resident_member<double>(bfvm_ctx*, bool);
+template bool resident_member<float>(bfvm_ctx*, bool);
+template cudaError_t run_resident_members<double>(bfvm_ctx* const*, int, bool, int, cudaStream_t);
+template cudaError_t run_resident_members<float>(bfvm_ctx* const*, int, bool, int, cudaStream_t);
 template int run_resident<double>(bfvm_ctx*, const SweepParams<double>&, const NodeLines&, bool, int, cudaStream_t,
                                   bool*);
 template int run_resident<float>(bfvm_ctx*, const SweepParams<float>&, const NodeLines&, bool, int, cudaStream_t,

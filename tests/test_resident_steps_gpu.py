@@ -34,9 +34,9 @@ def _run(wl, field, tmem, precision, chain, active, steps, plane=False, nodes=No
 # Line lengths about the batches of 16 values and the 8, 16 and 32 lanes of an
 # x row; last tiles of one line; face rows only (ny or nz of 1 and 2) and face
 # rows past 128 values; one tile and more than 148; eight warps to an SM, and
-# the first sizes past that; agents alone, many to a tile (more than 32) and
-# stacked in a voxel.
-SHAPES = [(3, 3, 3, 1, 9), (16, 16, 15, 2, 40), (17, 33, 31, 3, 3000), (31, 32, 48, 2, 500), (33, 47, 61, 7, 900),
+# the first sizes past that; agents alone, many to a tile (more than 32), so
+# many that they go ahead of the sweep, and stacked in a voxel.
+SHAPES = [(3, 3, 3, 1, 9), (16, 16, 15, 2, 40), (18, 9, 12, 2, 2000), (17, 33, 31, 3, 3000), (31, 32, 48, 2, 500), (33, 47, 61, 7, 900),
           (64, 64, 64, 9, 2000), (65, 1, 40, 2, 70), (1, 70, 33, 2, 60), (40, 2, 2, 2, 30), (200, 40, 33, 2, 4000),
           (129, 50, 7, 2, 100), (30, 300, 9, 1, 100), (100, 100, 96, 3, 2000)]
 
@@ -47,11 +47,11 @@ def test_resident_steps_equal_a_launch_per_stage(shape, precision, chain):
     nx, ny, nz, S, agents = shape
     wl = W.small_random(9000 + nx + ny + nz, nx=nx, ny=ny, nz=nz, S=S, n_agents=agents, steps=3)
     for active in (np.ones(S, np.uint8), np.arange(S, dtype=np.uint8) % 2):
-        a, b = (_run(wl, wl.field0, tmem, precision, chain, active, (1, 3)) for tmem in (1, 0))
+        a, b = (_run(wl, wl.field0, tmem, precision, chain, active, (1, 4)) for tmem in (1, 0))
         assert np.array_equal(a, b), (shape, precision, chain, active)
 
 
-@pytest.mark.parametrize("shape", [(1, 40, 1, 1, 20), (33, 16, 1, 2, 300), (90, 127, 1, 4, 500), (300, 61, 1, 2, 4000)])
+@pytest.mark.parametrize("shape", [(1, 40, 1, 1, 20), (33, 16, 1, 2, 300), (80, 33, 1, 2, 9000), (90, 127, 1, 4, 500), (300, 61, 1, 2, 4000)])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_resident_plane_steps_equal_a_launch_per_stage(shape, precision):
     nx, ny, nz, S, agents = shape
