@@ -23,7 +23,7 @@ namespace {
 // 128-byte lines, so the 16-byte loads are aligned; a row's last pair may end
 // in its padding, which is read and not written).  Bound by HBM; with one
 // voxel per thread of a flat index, a 64-bit division each, the pass took
-// BULK0 us at 160 x 200 x 120 x 3, now BULK1.
+// 83 us at 160 x 200 x 120 x 3, now 69.
 template <typename T>
 __global__ void __launch_bounds__(256) bulk_kernel(T* __restrict__ f, const double* __restrict__ rates, size_t plane,
                                                    int nx, int nxp, long long rows, int rows_per_s, double dt,

@@ -1094,7 +1094,7 @@ namespace {
 // Deterministic per-substrate sums: fixed block partials, then one block per
 // substrate adds them in a fixed tree.  A warp takes a row at a time, its
 // lanes along x (a 64-bit division per value and one thread adding all
-// partials had made the two launches SUM0 us at 160 x 200 x 120 x 3, now SUM1).
+// partials had made the two launches 42 + 50 us at 160 x 200 x 120 x 3, now 27 + 3).
 constexpr int kSumParts = 1024;
 
 // The block's sum of every thread's value, in thread 0.
