@@ -29,11 +29,13 @@
 //   300x260 2-D x3 FP64 50.7 -> 30.3 (49.4 -> 27.5); with 10,000 agents and a
 //                 rim of nodes 62.1 -> 43.7 (60.6 -> 41.2)
 // With one tile per warp it won at every size it takes, up to what an SM holds:
-// eight warps of 248 registers, or 227 KB of line buffers and coefficients.
+// eight warps of 254 registers, or 227 KB of line buffers and coefficients.
 // With several, the next tile's lines prefetched to the L2: see resident_wins;
-// 24 uneven FP32 solves of edges 24 to 128 (247 MB) 594 -> 425 us a step.
+// 24 uneven solves of edges 24 to 128: FP32 (247 MB) 594 -> 429 us a step, FP64
+// 932 -> 702.  Where it gives way to a launch per stage: resident_shares.
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <type_traits>
 
 #include "biofvm_b200.h"
@@ -960,29 +962,34 @@ cudaError_t launch_many(ResidentBatch<T, N>& b, int grid, size_t smem, int warps
 // 256x128x128 (three) 98 -> 70, 300x100x100 (two) 73 -> 75, 400x64x64x2 (two)
 // 81 -> 120.
 template <typename T>
+constexpr double kL2Share = sizeof(T) == 4 ? 1.0 : 0.55;
+
+template <typename T>
 bool resident_wins(const bfvm_ctx* c, const ResidentPlan& pl) {
   int l2 = 0;
   if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c->device) != cudaSuccess) return false;
   const double bytes = static_cast<double>(sizeof(T)) * c->nx * c->ny * c->nz * c->S;
-  return pl.warps >= 3 && bytes <= (sizeof(T) == 4 ? 1.0 : 0.55) * l2;
+  return pl.warps >= 3 && bytes <= kL2Share<T> * l2;
 }
 
 // And for a solve that has the GPU to itself or shares it with others on
 // streams of their own, which a launch per stage leaves more room for.  us per
 // call, FP32 unless stated, a launch per stage -> this, alone and three at once:
-//   64x64x64x8 (seven warps an SM): 1 step 37 -> 28 and 19 -> 24, 4 steps 143 ->
-//     78 and 71 -> 75, 10 steps 354 -> 178 and 177 -> 174; 50x50x50x2 FP64 (two
-//     warps) 1 step 32 -> 22 and 22 -> 10
-//   ten steps of 58x25x184x2 (five warps, their lanes 0.25 busy: 736 y tiles, 100
-//     z tiles) 391 -> 186 and 163 -> 182; 120x30x30x6 FP64 (0.46) 370 -> 175 and
-//     161 -> 172, 33x47x61x7 FP64 (0.50) 339 -> 173 and 170 -> 169; several tiles
-//     per warp: 58x25x184x4 (0.46) 411 -> 222 and 182 -> 218, 100x100x100x3 FP64
-//     (0.63) 702 -> 419 and 402 -> 416, 200x200x200x1 FP64 (0.70) 1357 -> 1027
-//     and 1111 -> 1034, 128x128x128x4 (0.99) 771 -> 511 and 547 -> 511
+//   two CTAs to an SM: 50x50x50x2 FP64 1 step 32 -> 22 and 22 -> 10, 10 steps
+//     309 -> 147 and 153 -> 54; 33x47x61x3 FP64 10 steps 319 -> 149 and 152 -> 80
+//   one: 64x64x64x8 (seven warps an SM) 1 step 37 -> 28 and 19 -> 24, 4 steps
+//     143 -> 78 and 71 -> 75, 10 steps 354 -> 178 and 177 -> 174
+//   ten steps by how busy the warps' lanes are: 58x25x184x2 (0.25: 736 y tiles,
+//     100 z tiles) 391 -> 186 and 163 -> 182, 150x24x24x3 FP64 (0.25) 370 -> 176
+//     and 153 -> 174, 120x30x30x6 FP64 (0.46) 370 -> 175 and 161 -> 172,
+//     33x47x61x7 FP64 (0.50) 339 -> 173 and 170 -> 169; several tiles per warp:
+//     58x25x184x4 (0.46) 411 -> 222 and 182 -> 218, 100x100x100x3 FP64 (0.63)
+//     702 -> 419 and 402 -> 416, 200x200x200x1 FP64 (0.70) 1357 -> 1027 and 1111
+//     -> 1034, 128x128x128x4 (0.99) 771 -> 511 and 547 -> 511
 //   with agents in 1 voxel of 17: 100x100x100x3 FP64 702 -> 499 and 437 -> 502,
 //     120x30x30x6 370 -> 205 and 163 -> 203: a tile takes them 32 at a time, a
 //     launch of its own with all threads
-// so more than four warps an SM come with four steps and more, agents in less
+// so runs whose CTAs fill an SM come with four steps and more, agents in less
 // than 1 voxel of 32, and lanes that are busy.
 template <typename T>
 bool resident_shares(const bfvm_ctx* c, const SweepParams<T>& p, const long long* tiles, long long warps, int nsteps,
@@ -1016,7 +1023,8 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
   unsigned long long* barrier = c->d_tile_counter + 4;
   if (resident_plan(c, p, nodes, two_d, false, sms, &pl, tiles, &smem)) {
     int grid = static_cast<int>(std::min<long long>(std::max(tiles[0], std::max(tiles[1], tiles[2])), sms));
-    if (pl.warps > 4 && !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.45))
+    if ((pl.warps > 4 || 2 * smem > kSmemMax) &&
+        !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.5))
       return BFVM_OK;
     int threads = 32 * pl.warps;
     if (pl.spread) {
@@ -1078,8 +1086,28 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
   ResidentBatch<T, kResidentMembers> b{};
   int sms = 0;
   if (count == 0 || sm_count(members[0]->device, &sms) != BFVM_OK) return cudaGetLastError();
+  // FP64 members go in launches of about equal bytes that stay in the L2 (what
+  // resident_wins asks of one): 24 of edges 24 to 128 (490 MB) 792 -> 700 us a
+  // step, 20 of edges to 110 421 -> 397; FP32's were as fast all at once (428
+  // and 436).
+  auto bytes = [&](int m) {
+    const bfvm_ctx* c = members[m];
+    return static_cast<double>(sizeof(T)) * c->nx * c->ny * c->nz * c->S;
+  };
+  int l2 = 0;
+  cudaError_t e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, members[0]->device);
+  if (e != cudaSuccess) return e;
+  double total = 0;
+  for (int m = 0; m < count; ++m) total += bytes(m);
+  const double share = total / std::ceil(total / (kL2Share<T> * l2));
   for (int m0 = 0; m0 < count; m0 += b.n) {
     b.n = std::min(count - m0, std::min(kResidentMembers, sms));
+    if (sizeof(T) == 8) {
+      double taken = 0;
+      int k = 0;
+      for (; k < b.n && (k == 0 || taken + 0.5 * bytes(m0 + k) <= share); ++k) taken += bytes(m0 + k);
+      b.n = k;
+    }
     long long tiles[kResidentMembers][3];
     size_t smem = 0;
     int warps = 0;
@@ -1121,7 +1149,7 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
           resident_spreads(members[m0 + m], b.solve[m].p, (tiles[m][0] + w - 1) / w, 32ll * warps * b.solve[m].ctas) ? 1 : 0;
       cta += b.solve[m].ctas;
     }
-    const cudaError_t e = launch_many(b, grid, smem, warps, nsteps, st);
+    e = launch_many(b, grid, smem, warps, nsteps, st);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
