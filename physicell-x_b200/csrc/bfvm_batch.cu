@@ -127,10 +127,20 @@ int build_tables(bfvm_batch* b, bool sources) {
   b->batched = false;
   b->direct_launches = 0;
   b->resident_launches = 0;
+  // Dense agents cost the one launch more than a launch per stage, whose
+  // threads all take them: 10 FP64 members of edges to 55 with agents in 1 voxel
+  // of 6, six steps, 466 -> 378 us a call alone, but 247 -> 308 for each of three
+  // batches at once.
+  long long voxels = 0, agents = 0;
+  for (const bfvm_ctx* c : b->members) {
+    voxels += 1LL * c->nx * c->ny * c->nz;
+    agents += c->n_agents;
+  }
+  const bool sparse = !sources || 32 * agents <= voxels;
   for (int q = 0; q < n; ++q) {
     bfvm_ctx* c = b->members[q];
     const bool direct = b->mode == 2 && 1LL * c->nx * c->ny * c->nz * c->S >= b->direct_min;
-    const bool resident = b->mode == 2 && resident_member<T>(c, sources);
+    const bool resident = b->mode == 2 && sparse && resident_member<T>(c, sources);
     if (resident) b->resident.push_back(c);
     if (resident && !direct) b->batched = true;
     if (direct) {

@@ -506,24 +506,54 @@ __device__ __forceinline__ void resident_sources(const SweepParams<T>& p, const 
 }
 
 // The sources by all of the run's threads, thread `id` of `threads`, ahead of
-// the x sweep and a barrier: where many agents lie in a tile.
+// the x sweep and a barrier: where many agents lie in a tile.  Four agents a
+// thread at a time, two memory latencies for the four.
 template <typename T>
-__device__ __forceinline__ void resident_spread(const SweepParams<T>& p, long long id, long long threads) {
+__device__ __forceinline__ void resident_spread(const SweepParams<T>& p, unsigned id, unsigned threads) {
+  constexpr int kAgents = 4;
   const int rows = p.ny * p.nz, n = __ldg(p.line_off + rows);
-  for (long long e = id; e < static_cast<long long>(n) * p.S; e += threads) {
-    const int s = static_cast<int>(e / n), q = static_cast<int>(e - static_cast<long long>(s) * n);
-    const unsigned key = __ldg(p.a_key + q), before = __ldg(p.a_key + max(q - 1, 0));
-    const size_t sn = static_cast<size_t>(s) * p.n_sorted;
-    const double k1 = __ldg(p.ac1 + sn + q), k2 = __ldg(p.ac2 + sn + q), k3 = __ldg(p.ae2 + sn + q);
-    if (q > 0 && before == key) continue;
-    const int row = static_cast<int>(key / p.nx), i = static_cast<int>(key - static_cast<unsigned>(row) * p.nx);
-    const int k = row / p.ny, j = row - k * p.ny;
-    if (p.active[s] != 0 && (j == 0 || j == p.ny - 1 || k == 0 || k == p.nz - 1)) continue;
-    T* const rho = p.f + (static_cast<size_t>(s) * rows + row) * p.nxp + i;
-    T x = __ldcg(rho);
-    apply_run<T>(&x, q, key, k1, k2, k3, n, p.a_key, p.ac1 + sn, p.ac2 + sn, p.ae2 + sn,
-                 sizeof(T) == 4 ? p.off[s] : 0.0, s, p.track);
-    *rho = x;
+  const unsigned total = static_cast<unsigned>(n) * p.S;  // (below 2^31: resident_spreads)
+  for (unsigned e0 = id; e0 < total; e0 += kAgents * threads) {
+    unsigned key[kAgents], before[kAgents], after[kAgents];
+    double k1[kAgents], k2[kAgents], k3[kAgents];
+    T* rho[kAgents];
+    T x[kAgents];
+#pragma unroll
+    for (int u = 0; u < kAgents; ++u) {
+      const unsigned e = min(e0 + u * threads, total - 1);
+      const int s = static_cast<int>(e / n), q = static_cast<int>(e - s * n);
+      const size_t at = static_cast<size_t>(s) * p.n_sorted + q;
+      key[u] = __ldg(p.a_key + q);
+      before[u] = __ldg(p.a_key + max(q - 1, 0));
+      after[u] = __ldg(p.a_key + min(q + 1, n - 1));
+      k1[u] = __ldg(p.ac1 + at);
+      k2[u] = __ldg(p.ac2 + at);
+      k3[u] = __ldg(p.ae2 + at);
+    }
+#pragma unroll
+    for (int u = 0; u < kAgents; ++u) {
+      const unsigned e = e0 + u * threads;
+      const int s = static_cast<int>(e / n), q = static_cast<int>(e - s * n);
+      const int row = static_cast<int>(key[u] / p.nx), i = static_cast<int>(key[u] - static_cast<unsigned>(row) * p.nx);
+      const int k = row / p.ny, j = row - k * p.ny;
+      rho[u] = nullptr;
+      x[u] = T(0);
+      if (e >= total || (q > 0 && before[u] == key[u]) ||
+          (p.active[s] != 0 && (j == 0 || j == p.ny - 1 || k == 0 || k == p.nz - 1)))
+        continue;
+      rho[u] = p.f + (static_cast<size_t>(s) * rows + row) * p.nxp + i;
+      x[u] = __ldcg(rho[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kAgents; ++u) {
+      if (rho[u] == nullptr) continue;
+      const unsigned e = e0 + u * threads;
+      const int s = static_cast<int>(e / n), q = static_cast<int>(e - s * n);
+      const size_t sn = static_cast<size_t>(s) * p.n_sorted;
+      apply_run<T>(&x[u], q, key[u], k1[u], k2[u], k3[u], q + 1 < n && after[u] == key[u] ? n : q + 1, p.a_key,
+                   p.ac1 + sn, p.ac2 + sn, p.ae2 + sn, sizeof(T) == 4 ? p.off[s] : 0.0, s, p.track);
+      *rho[u] = x[u];
+    }
   }
 }
 
@@ -743,7 +773,7 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   GridBarrier bar{barrier, gridDim.x};
   for (int step = 0; step < pl.nsteps; ++step) {
     if (pl.spread) {
-      resident_spread(p, w0 * 32ll + (threadIdx.x & 31), nw * 32ll);
+      resident_spread(p, w0 * 32 + (threadIdx.x & 31), nw * 32);
       if (!bar.sync(p.status)) break;
     }
     resident_tile<T, 0>(
@@ -821,8 +851,7 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1) resident_many_kernel(co
   for (int step = 0; step < b.nsteps; ++step) {
     for (int q = w0; q < pl.face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
     if (pl.spread) {
-      resident_spread(p, static_cast<long long>(blockIdx.x - b.solve[m].cta0) * blockDim.x + threadIdx.x,
-                      static_cast<long long>(ctas) * blockDim.x);
+      resident_spread(p, (blockIdx.x - b.solve[m].cta0) * blockDim.x + threadIdx.x, ctas * blockDim.x);
       if (!bar.sync(p.status)) break;
     }
     for (int tile = w0; tile < ntx; tile += nw) {
@@ -854,14 +883,15 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1) resident_many_kernel(co
 // Whether the sources go ahead of the x sweep, spread over `threads` threads.
 // x tiles take them 32 at a time, about 1,000 cycles (an exact division, then
 // the runs of stacked agents), `rounds` tiles one after another; the spread
-// phase takes a barrier and about 2,000 cycles for each agent of a thread.
-// us per step, FP64, 10 steps, in the tiles -> spread: a plane of 537x74x3 with
-// 2,000 agents (20 rounds) 41 -> 33, with 8,000 (83) 100 -> 34; 200x200x200x1
-// with 1.6 million (3 x 40 rounds, 42 spread) 250 -> 182; but 64x64x64x8 FP32
-// with 52,000 (13 rounds, 11 spread) 25 -> 36.
+// phase takes a barrier and up to 2,000 cycles for each agent of a thread.
+// us per step, FP64, 10 steps, in the tiles -> spread: a plane of 300x260x3 with
+// 10,000 agents and a rim of nodes 63 -> 41, of 537x74x3 with 8,000 (83 rounds)
+// 100 -> 37; 200x200x200x1 with 1.6 million (3 x 40 rounds, 42 spread) 250 -> 182;
+// but 64x64x64x8 FP32 with 52,000 (13 rounds, 11 spread) 25 -> 36, and spread at
+// half these lines 24 uneven FP32 solves side by side 427 -> 470.
 template <typename T>
 bool resident_spreads(const bfvm_ctx* c, const SweepParams<T>& p, long long rounds, long long threads) {
-  if (p.line_off == nullptr) return false;
+  if (p.line_off == nullptr || static_cast<long long>(c->n_agents) * c->S > INT_MAX / 2) return false;
   const long long tiles = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
   const long long in_tiles = rounds * ((c->n_agents / tiles + 31) / 32);
   return in_tiles > 8 + 2 * ((static_cast<long long>(c->n_agents) * c->S + threads - 1) / threads);
@@ -989,8 +1019,8 @@ bool resident_wins(const bfvm_ctx* c, const ResidentPlan& pl) {
 //   with agents in 1 voxel of 17: 100x100x100x3 FP64 702 -> 499 and 437 -> 502,
 //     120x30x30x6 370 -> 205 and 163 -> 203: a tile takes them 32 at a time, a
 //     launch of its own with all threads
-// so runs whose CTAs fill an SM come with four steps and more, agents in less
-// than 1 voxel of 32, and lanes that are busy.
+// so runs that leave no room for another come with four steps and more, agents
+// in less than 1 voxel of 32, and lanes that are busy.
 template <typename T>
 bool resident_shares(const bfvm_ctx* c, const SweepParams<T>& p, const long long* tiles, long long warps, int nsteps,
                      double busy) {
@@ -1023,9 +1053,6 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
   unsigned long long* barrier = c->d_tile_counter + 4;
   if (resident_plan(c, p, nodes, two_d, false, sms, &pl, tiles, &smem)) {
     int grid = static_cast<int>(std::min<long long>(std::max(tiles[0], std::max(tiles[1], tiles[2])), sms));
-    if ((pl.warps > 4 || 2 * smem > kSmemMax) &&
-        !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.5))
-      return BFVM_OK;
     int threads = 32 * pl.warps;
     if (pl.spread) {
       // Eight agents a thread, and two CTAs to an SM where their lines allow it:
@@ -1035,6 +1062,10 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
       grid = static_cast<int>(std::max<long long>(grid, std::min<long long>(ctas, sms)));
       threads = std::max(threads, kSpreadThreads);
     }
+    // whether another such run finds room beside this one: 227 KB and eight warps an SM
+    const long long per_sm = std::min<long long>(kSmemMax / smem, kResidentWarps / std::max(pl.warps, threads / 32));
+    if (2 * grid > per_sm * sms && !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.5))
+      return BFVM_OK;
     int blocks = 0;
     BFVM_CUDA(persistent_grid(resident_kernel<T>, smem, grid, &blocks, threads));
     if (blocks < grid) return BFVM_OK;

@@ -72,7 +72,7 @@ def test_batch_members_side_by_side_equal_solves_alone(precision, members):
     and of more than the batch's graph, and of more than one launch takes."""
     rng = np.random.default_rng(members)
     wls = [W.small_random(40 + q, nx=int(rng.integers(1, 60)), ny=int(rng.integers(1, 60)), nz=int(rng.integers(2, 60)),
-                          S=int(rng.integers(1, 7)), n_agents=int(rng.integers(1, 3000)), steps=1)
+                          S=int(rng.integers(1, 7)), n_agents=int(rng.integers(1, 600)), steps=1)
            for q in range(members)]
     for tracked in (False, True):
         batch, mes = Batch(precision), []
