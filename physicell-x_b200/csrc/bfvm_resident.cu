@@ -208,8 +208,9 @@ __device__ __forceinline__ void resident_tile(const SweepParams<T>& p, const Res
   const int s = l.s;
   const bool act = l.act, on = l.on, fast = p.screen == kScreenFast;
   const double c1 = l.c1, shift = l.shift, x0 = l.x0, x1 = l.x1;
-  const DR* dr = reinterpret_cast<const DR*>(coef + pl.dr_off[AXIS]) + (pl.own ? 0 : static_cast<size_t>(s) * pl.rows[AXIS]);
-  const double* cu = coef + pl.cu_off[AXIS] + (pl.own ? 0 : static_cast<size_t>(s) * pl.rows[AXIS]);
+  const size_t set = pl.own ? 0 : static_cast<size_t>(s) * pl.rows[AXIS];
+  const DR* dr = reinterpret_cast<const DR*>(coef + pl.dr_off[AXIS]) + set;
+  const double* cu = coef + pl.cu_off[AXIS] + set;
 
   // ---- the tile in: every copy under way at once (one memory latency for
   // the tile, 1,200 cycles), 16 bytes a lane (8 took three times as long for
@@ -689,7 +690,8 @@ __device__ __forceinline__ void resident_prefetch(const SweepParams<T>& p, int t
     const int nm = AXIS == 1 ? p.nz : p.ny, n = AXIS == 1 ? p.ny : p.nz;
     const int xt = (p.nx + 31) / 32, per_s = xt * nm, s = tile / per_s, q = tile - s * per_s, m = q / xt;
     const size_t stride = resident_stride<T, AXIS>(p);
-    at = p.f + (AXIS == 1 ? (static_cast<size_t>(s) * p.nz + m) * p.ny : static_cast<size_t>(s) * p.nz * p.ny + m) * p.nxp +
+    const size_t plane = static_cast<size_t>(s) * p.nz, row = AXIS == 1 ? (plane + m) * p.ny : plane * p.ny + m;
+    at = p.f + row * p.nxp +
          (q - m * xt) * 32 + t / kLines * stride + t % kLines * kLine;
     step = 32 / kLines * stride;
     count = n * kLines;
@@ -824,7 +826,8 @@ template <typename T>
 constexpr int kManyWarps = sizeof(T) == 4 ? 12 : 8;
 
 template <typename T, int N>
-__global__ void __launch_bounds__(32 * kManyWarps<T>, 1) resident_many_kernel(const __grid_constant__ ResidentBatch<T, N> b) {
+__global__ void __launch_bounds__(32 * kManyWarps<T>, 1)
+    resident_many_kernel(const __grid_constant__ ResidentBatch<T, N> b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   int m = 0;
   if constexpr (N > 1) {
@@ -840,7 +843,8 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1) resident_many_kernel(co
   const int w0 = warp < pl.warps ? static_cast<int>(blockIdx.x) - b.solve[m].cta0 + ctas * warp : INT_MAX / 2;
   unsigned char* const keep = smem_raw + static_cast<size_t>(warp) * pl.warp_bytes;
   T* const buf = reinterpret_cast<T*>(keep);
-  double* const agents = reinterpret_cast<double*>(keep + static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T));
+  double* const agents =
+      reinterpret_cast<double*>(keep + static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T));
   const int pitch = resident_pitch<T>(p.nx);
   const int xt = (p.nx + 31) / 32;
   const int ntx = (p.ny * p.nz + 31) / 32 * p.S, nty = xt * p.nz * p.S, ntz = xt * p.ny * p.S;
@@ -1058,7 +1062,8 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
       // Eight agents a thread, and two CTAs to an SM where their lines allow it:
       // a small grid leaves SMs to others' work (600x500x4 FP32 with 18,000
       // agents, 10 steps, three solves at once: 469 us a call on all SMs).
-      const long long ctas = (static_cast<long long>(c->n_agents) * c->S + 8 * kSpreadThreads - 1) / (8 * kSpreadThreads);
+      const long long ctas =
+          (static_cast<long long>(c->n_agents) * c->S + 8 * kSpreadThreads - 1) / (8 * kSpreadThreads);
       grid = static_cast<int>(std::max<long long>(grid, std::min<long long>(ctas, sms)));
       threads = std::max(threads, kSpreadThreads);
     }
@@ -1177,7 +1182,9 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
       b.solve[m].cta0 = cta;
       const long long w = static_cast<long long>(b.solve[m].ctas) * b.solve[m].pl.warps;
       b.solve[m].pl.spread =
-          resident_spreads(members[m0 + m], b.solve[m].p, (tiles[m][0] + w - 1) / w, 32ll * warps * b.solve[m].ctas) ? 1 : 0;
+          resident_spreads(members[m0 + m], b.solve[m].p, (tiles[m][0] + w - 1) / w, 32ll * warps * b.solve[m].ctas)
+              ? 1
+              : 0;
       cta += b.solve[m].ctas;
     }
     e = launch_many(b, grid, smem, warps, nsteps, st);
