@@ -41,6 +41,7 @@
 #include "biofvm_b200.h"
 #include "bfvm_ctx.h"
 #include "bfvm_internal.h"
+#include "bfvm_prefetch_lines.h"
 #include "bfvm_ptx.cuh"
 #include "bfvm_sweep_common.cuh"
 
@@ -676,27 +677,9 @@ template <typename T, int AXIS>
 __device__ __forceinline__ void resident_prefetch(const SweepParams<T>& p, int tile, int tiles) {
   if (tile >= tiles) return;
   const int t = threadIdx.x & 31;
-  constexpr int kLine = 128 / sizeof(T);
-  const T* at;
-  size_t step;
-  int count;
-  if (AXIS == 0) {
-    const int rows = p.ny * p.nz, per_s = (rows + 31) / 32, s = tile / per_s, r0 = (tile - s * per_s) * 32;
-    at = p.f + (static_cast<size_t>(s) * rows + r0) * p.nxp + t * kLine;
-    step = 32 * kLine;
-    count = min(32, rows - r0) * (p.nxp / kLine);
-  } else {
-    constexpr int kLines = 32 / kLine;  // per row
-    const int nm = AXIS == 1 ? p.nz : p.ny, n = AXIS == 1 ? p.ny : p.nz;
-    const int xt = (p.nx + 31) / 32, per_s = xt * nm, s = tile / per_s, q = tile - s * per_s, m = q / xt;
-    const size_t stride = resident_stride<T, AXIS>(p);
-    const size_t plane = static_cast<size_t>(s) * p.nz, row = AXIS == 1 ? (plane + m) * p.ny : plane * p.ny + m;
-    at = p.f + row * p.nxp +
-         (q - m * xt) * 32 + t / kLines * stride + t % kLines * kLine;
-    step = 32 / kLines * stride;
-    count = n * kLines;
-  }
-  for (int q = t; q < count; q += 32, at += step) asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+  const PrefetchLines l = prefetch_lines<AXIS, 128 / static_cast<int>(sizeof(T))>(p.nx, p.ny, p.nz, p.nxp, tile, t);
+  const T* at = p.f + l.at;
+  for (int q = t; q < l.count; q += 32, at += l.step) asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
 }
 
 // A run's coefficients to shared memory, every copy under way at once (a plane's
