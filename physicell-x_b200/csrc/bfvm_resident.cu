@@ -94,7 +94,7 @@ struct ResidentPlan {
   int line;       // values of the longest line: sizes a warp's buffer
   int nsteps;
   int two_d;
-  int face_rows;  // y and z face lines of all activated substrates
+  int face_rows;  // y and z face lines of one activated substrate
   int dr_off[3];  // staged coefficient rows of each axis, in doubles from the coefficients' start
   int cu_off[3];
   int rows[3];    // rows per substrate of each axis
@@ -559,6 +559,20 @@ __device__ __forceinline__ void resident_spread(const SweepParams<T>& p, unsigne
   }
 }
 
+// The face lines of all activated substrates.  How many are activated is read
+// when the launch runs: a captured launch outlives the activation it was
+// captured under, and the lines it leaves out of the sweeps follow the device's.
+template <typename T>
+__device__ __forceinline__ int resident_face_rows(const SweepParams<T>& p, const ResidentPlan& pl) {
+  if (pl.face_rows == 0) return 0;
+  int on = 0;
+  for (int s0 = 0; s0 < p.S; s0 += 32) {
+    const int s = s0 + (threadIdx.x & 31);
+    on += __popc(__ballot_sync(0xffffffffu, s < p.S && p.active[s] != 0));
+  }
+  return on * pl.face_rows;
+}
+
 // The y and z face lines of activated substrates take their face's values
 // (their ends, the x faces') in the x sweep's place: row number `at` of all
 // of them, by one warp, coalesced.
@@ -750,8 +764,9 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   const ResidentNodes<T> yn = resident_nodes(p, nd, 1, w0, pl.nodes[1], keep);
   const int l0 = w0 % ((p.ny + 31) / 32) * 32;  // (of a plane)
   __syncwarp();
+  const int face_rows = resident_face_rows(p, pl);
   ResidentFace<T> face{};
-  if (w0 < pl.face_rows) face = resident_face(p, w0);
+  if (w0 < face_rows) face = resident_face(p, w0);
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const auto none = [] {};
@@ -771,7 +786,7 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
           if (xn.n > 0) resident_pin(p, xn, false, buf, pitch, l0);
         });
     resident_face_store(face, p.nx);
-    for (int q = w0 + nw; q < pl.face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
+    for (int q = w0 + nw; q < face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
     if (!bar.sync(p.status)) break;
     resident_tile<T, 1>(p, pl, coef, buf, ly, none, none, none);
     if (yn.n > 0) resident_pin<T>(p, yn, true, nullptr, 0, 0);
@@ -830,13 +845,14 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1)
       reinterpret_cast<double*>(keep + static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T));
   const int pitch = resident_pitch<T>(p.nx);
   const int xt = (p.nx + 31) / 32;
+  const int face_rows = resident_face_rows(p, pl);
   const int ntx = (p.ny * p.nz + 31) / 32 * p.S, nty = xt * p.nz * p.S, ntz = xt * p.ny * p.S;
   asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
   const auto none = [] {};
   GridBarrier bar{b.solve[m].barrier, static_cast<unsigned>(ctas)};
   for (int step = 0; step < b.nsteps; ++step) {
-    for (int q = w0; q < pl.face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
+    for (int q = w0; q < face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
     if (pl.spread) {
       resident_spread(p, (blockIdx.x - b.solve[m].cta0) * blockDim.x + threadIdx.x, ctas * blockDim.x);
       if (!bar.sync(p.status)) break;
@@ -898,10 +914,8 @@ bool resident_plan(const bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& 
   ResidentPlan pl{};
   pl.two_d = two_d ? 1 : 0;
   if (!two_d) {
-    int on = 0;
-    for (int s = 0; s < S; ++s) on += c->active[s] ? 1 : 0;
     const int zrows = (c->nz > 1 ? 2 : 1) * c->ny, yrows = (c->ny > 1 ? 2 : 1) * (c->nz > 2 ? c->nz - 2 : 0);
-    pl.face_rows = on * (zrows + yrows);
+    pl.face_rows = zrows + yrows;
   }
   const long long xt = (c->nx + 31) / 32, xrows = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
   tiles[0] = xrows * S;
