@@ -61,9 +61,11 @@ struct bfvm_batch {
   size_t axis_smem[3] = {0, 0, 0};
   bool built_sources = false;
   // The device tables are rebuilt only when the membership, the schedule, the
-  // sources flag or a member's device pointers (bfvm_ctx::version) changed.
+  // sources flag, a member's device pointers (bfvm_ctx::version) or, where
+  // members take different forms, its launch settings (bfvm_ctx::settings)
+  // changed.
   bool dirty = true;
-  std::vector<int> versions;
+  std::vector<int> versions;  // table_version of each member
   // captured graph of graph_steps steps
   cudaGraphExec_t gexec = nullptr;
   size_t g_smem = 0;
@@ -385,17 +387,20 @@ int release_members(bfvm_batch* b) {
   return BFVM_OK;
 }
 
+// (a sum of two counts that only grow)
+int table_version(const bfvm_batch* b, const bfvm_ctx* c) { return c->version + (b->mode == 2 ? c->settings : 0); }
+
 template <typename T>
 int step_impl(bfvm_batch* b, int nsteps, bool sources) {
   if (b->members.empty() || nsteps == 0) return BFVM_OK;
   int rc = join_members(b);
   if (rc != BFVM_OK) return rc;
   bool rebuild = b->dirty || sources != b->built_sources || b->versions.size() != b->members.size();
-  for (size_t q = 0; !rebuild && q < b->members.size(); ++q) rebuild = b->versions[q] != b->members[q]->version;
+  for (size_t q = 0; !rebuild && q < b->members.size(); ++q) rebuild = b->versions[q] != table_version(b, b->members[q]);
   if (rebuild) {
     if ((rc = build_tables<T>(b, sources)) != BFVM_OK) return rc;
     b->versions.resize(b->members.size());
-    for (size_t q = 0; q < b->members.size(); ++q) b->versions[q] = b->members[q]->version;
+    for (size_t q = 0; q < b->members.size(); ++q) b->versions[q] = table_version(b, b->members[q]);
     b->dirty = false;
   }
   int left = nsteps;

@@ -1199,9 +1199,17 @@ extern "C" int bfvm_set_wait_limit_ns(int device, unsigned long long ns) {
   return BFVM_OK;
 }
 
+// A launch setting's new value.  A batch that the solve belongs to decides with
+// its tables which form each member takes: it builds them again.
+template <typename V>
+static void change_setting(bfvm_ctx* c, V* setting, V value) {
+  if (*setting != value) ++c->settings;
+  *setting = value;
+}
+
 extern "C" int bfvm_timing_enable(bfvm_ctx* c, int on) {
   if (!c) return BFVM_ERR_ARG;
-  c->timing = on != 0;
+  change_setting(c, &c->timing, on != 0);
   return BFVM_OK;
 }
 
@@ -1346,7 +1354,7 @@ extern "C" int bfvm_set_sweep_schedule(bfvm_ctx* c, int persistent) {
   if (!c || persistent < 0 || persistent > 2) return BFVM_ERR_ARG;
   DeviceGuard g(c->device);
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
-  c->cfg.persistent = persistent;
+  change_setting(c, &c->cfg.persistent, persistent);
   return BFVM_OK;
 }
 
@@ -1354,7 +1362,7 @@ extern "C" int bfvm_set_substrate_streams(bfvm_ctx* c, int streams) {
   if (!c || (streams != 1 && streams != 2)) return BFVM_ERR_ARG;
   DeviceGuard g(c->device);
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
-  c->sub_streams = streams;  // part of the step graph's key: recaptured on the next run
+  change_setting(c, &c->sub_streams, streams);  // part of the step graph's key: recaptured on the next run
   return BFVM_OK;
 }
 
@@ -1368,7 +1376,7 @@ extern "C" int bfvm_set_fused_sources(bfvm_ctx* c, int fused) {
   if (!c || (fused != 0 && fused != 1)) return BFVM_ERR_ARG;
   DeviceGuard g(c->device);
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
-  c->cfg.fuse_sources = fused;
+  change_setting(c, &c->cfg.fuse_sources, fused);
   return BFVM_OK;
 }
 
@@ -1401,7 +1409,7 @@ extern "C" int bfvm_set_partition_min_line(bfvm_ctx* c, int n_line) {
   if (!c || n_line < -1 || n_line == 0) return BFVM_ERR_ARG;
   DeviceGuard g(c->device);
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
-  c->part_min_line = n_line;
+  change_setting(c, &c->part_min_line, n_line);
   return BFVM_OK;
 }
 
@@ -1415,7 +1423,7 @@ extern "C" int bfvm_set_sweep_tmem(bfvm_ctx* c, int on) {
   if (!c || on < 0 || on > 2) return BFVM_ERR_ARG;
   DeviceGuard g(c->device);
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
-  c->cfg.tmem = on;
+  change_setting(c, &c->cfg.tmem, on);
   return BFVM_OK;
 }
 
@@ -1456,6 +1464,7 @@ extern "C" int bfvm_set_launch(bfvm_ctx* c, int x_lines, int yz_tile, int yz_chu
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
   c->maps = maps;
   c->cfg = cfg;
+  ++c->settings;
   return BFVM_OK;
 }
 

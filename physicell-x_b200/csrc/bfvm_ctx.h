@@ -95,6 +95,7 @@ struct bfvm_ctx {
   size_t device_bytes = 0;     // bytes currently allocated by dalloc
   std::unordered_map<void*, size_t> alloc_bytes;
   int version = 0;             // bumped whenever device pointers in SweepParams change
+  int settings = 0;            // bumped whenever a launch setting changes, and with it the form a step may take
   double* d_staging = nullptr; // reference-layout field, for host uploads/downloads
   double* d_grad = nullptr;    // gradients for host reads (bfvm_compute_gradients)
   double* d_bulk = nullptr;    // bulk supply | target | uptake rates, device layout (bfvm_set_bulk_rates)

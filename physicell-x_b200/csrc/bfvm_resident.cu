@@ -1131,7 +1131,11 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
   cudaError_t e = cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, members[0]->device);
   if (e != cudaSuccess) return e;
   double total = 0;
-  for (int m = 0; m < count; ++m) total += bytes(m);
+  for (int m = 0; m < count; ++m) {
+    // all or none: what some members' launches took would be steps ahead
+    if (!resident_member<T>(members[m], sources)) return cudaErrorInvalidValue;
+    total += bytes(m);
+  }
   const double share = total / std::ceil(total / (kL2Share<T> * l2));
   for (int m0 = 0; m0 < count; m0 += b.n) {
     b.n = std::min(count - m0, std::min(kResidentMembers, sms));

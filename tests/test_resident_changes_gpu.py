@@ -81,3 +81,43 @@ def test_captured_run_follows_the_activation(shape, precision):
     del graph
     me.close()
     solo.close()
+
+
+SETTINGS = {
+    "timing": lambda me, on: me.timing_enable(not on),
+    "tmem": lambda me, on: me.set_sweep_tmem(1 if on else 0),
+    "schedule": lambda me, on: me.set_sweep_schedule(1 if on else 2),
+    "streams": lambda me, on: me.set_substrate_streams(1 if on else 2),
+    "launch": lambda me, on: me.set_launch(32 if on else 64, 32, 32),
+    "fused": lambda me, on: me.set_fused_sources(not on),
+    "chain": lambda me, on: me.set_fp64_chain(0 if on else 1),
+}
+
+
+@pytest.mark.parametrize("setting", sorted(SETTINGS))
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_batch_follows_its_members_settings(setting, precision):
+    """A member's launch setting changes between the steps of a batch and goes
+    back: the member leaves the one launch or returns to it, and every member
+    goes on step by step, in calls that replay the graph and in ones that do
+    not.  50 members: the one launch is two."""
+    wls = [W.small_random(990 + q, nx=9 + q % 7, ny=8 + q % 5, nz=7 + q % 3, S=2, n_agents=20, steps=1)
+           for q in range(50)]
+    batch = Batch(precision)
+    batch.set_schedule(mode=2, graph_steps=4)
+    mes, solos = ([_solve(wl, precision, tmem) for wl in wls] for tmem in (1, 0))
+    for me in mes:
+        batch.add(me)
+    for on in (True, False, True):
+        SETTINGS[setting](mes[-1], on)
+        if setting == "chain":
+            SETTINGS[setting](solos[-1], on)
+        for n in (2, 4):
+            batch.step(n, sources=True)
+        batch.synchronize()
+        for q, (me, solo) in enumerate(zip(mes, solos)):
+            solo.simulate_diffusion_decay(6, sources=True)
+            assert np.array_equal(me.download_field(), solo.download_field()), (q, on)
+    batch.close()
+    for me in mes + solos:
+        me.close()
