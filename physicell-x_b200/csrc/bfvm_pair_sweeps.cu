@@ -42,6 +42,7 @@
 
 #include "biofvm_b200.h"
 #include "bfvm_internal.h"
+#include "bfvm_pair_coefs.h"
 #include "bfvm_ptx.cuh"
 #include "bfvm_sweep_common.cuh"
 
@@ -65,7 +66,8 @@ struct PairPlan {
   int C;      // chunks per line
   int rings;  // compute warps 0 .. rings-1; the CTA's second half of warps copies for them
   int D;      // slots of a ring (<= C)
-  int KC;     // staged coefficient chunks a ring has room for
+  int KC;     // staged coefficient chunks a ring has room for,
+  int conv;   // for lines whose rows are constant from this entry on
   int pw;     // packed partial tiles of the y/z sweeps (FieldMaps::pyz_w)
   int TU;     // units of a ring in TMEM; the other C - TU in shared memory
   uint32_t ring_bytes;
@@ -350,30 +352,18 @@ __device__ __forceinline__ void pair_compute(const SweepParams<T>& p, const Pair
   const int pw = pl.pw, pw_log = pw > 0 ? 31 - __clz(pw) : 0;
 
   // ---- coefficient rows, staged per substrate ----
-  // Chunks k0 .. k1 hold one and the same pair of rows (the
-  // factorization's fixed point, AxisCoefs::conv) and are staged once.
-  struct Conv {
-    int k0, k1;  // none: k0 > k1
-    __device__ __forceinline__ int sh() const { return max(k1 - k0, 0); }
-    __device__ __forceinline__ int at(int c) const { return c < k0 ? c : max(k0, c - sh()); }
-  };
   const AxisCoefs<T>& ac = X ? p.ax : (AXIS == 1 ? p.ay : p.az);
   auto conv_of = [&](int s) {
-    Conv v{C, C - 1};
-    if (ac.conv != nullptr && n >= 3) {
-      const int k0 = (__ldg(ac.conv + s) + R - 1) / R, k1 = (n - 1) / R - 1;  // chunks ending at n - 2 or before
-      if (k1 >= k0) v = Conv{k0, k1};
-    }
-    return v;
+    return pair_conv(C, R, n, ac.conv != nullptr ? __ldg(ac.conv + s) : n, pl.conv);
   };
-  auto stage_chunks = [&](auto* dst, const auto* src, const Conv& cv) {
+  auto stage_chunks = [&](auto* dst, const auto* src, const PairConv& cv) {
     const int sh = cv.sh(), m = (C - sh) * R;
     __syncwarp();
     for (int q = t; q < m; q += 32) dst[q] = __ldg(src + q + (q / R > cv.k0 ? sh * R : 0));
     __syncwarp();
   };
   int dr_s = -1, cu_s = -1;
-  Conv dr_cv{0, C}, cu_cv{0, C};  // before the first tile: chunk 0 throughout
+  PairConv dr_cv{0, C}, cu_cv{0, C};  // before the first tile: chunk 0 throughout
   DR dk{};          // B's converged forward coefficients
   double ck = 0.0;  // A's converged upper diagonal
 
@@ -903,8 +893,8 @@ static bool pair_plan(int n, int conv_max, int pw, PairPlan* out) {
   PairPlan pl{};
   pl.C = (n + F::R - 1) / F::R;
   pl.pw = pw;
-  const int k0 = (conv_max + F::R - 1) / F::R, k1 = (n - 1) / F::R - 1;
-  pl.KC = pl.C - (n >= 3 && k1 > k0 ? k1 - k0 : 0);
+  pl.conv = conv_max;
+  pl.KC = pl.C - pair_conv(pl.C, F::R, n, conv_max).sh();
   const int rq = pl.C <= 256 / F::kCols ? 2 : 1;
   pl.TU = pl.C < 512 / rq / F::kCols ? pl.C : 512 / rq / F::kCols;
   for (pl.rings = 4 * rq; pl.rings >= 1; --pl.rings) {

@@ -5,11 +5,7 @@
 // against the field's extent.
 #pragma once
 
-#ifdef __CUDACC__
-#define BFVM_HD __host__ __device__ __forceinline__
-#else
-#define BFVM_HD inline
-#endif
+#include "bfvm_host_device.h"
 
 namespace bfvm {
 
