@@ -104,6 +104,7 @@ struct ResidentPlan {
   int agents, nodes[2];
   int own;     // one warp: the coefficients of its own tiles' substrates only
   int spread;  // the sources ahead of the x sweep, by every thread of the run
+  int crowd;   // so too where some x tile holds more agents than this
   int warp_bytes;  // (a multiple of 16, as each list is)
 };
 
@@ -573,6 +574,20 @@ __device__ __forceinline__ int resident_face_rows(const SweepParams<T>& p, const
   return on * pl.face_rows;
 }
 
+// Whether some x tile that this thread looks at holds more than pl.crowd agents
+// (the threads of a CTA look at all of them between them, so every CTA of the
+// run comes to the same answer).
+template <typename T>
+__device__ __forceinline__ bool resident_crowded(const SweepParams<T>& p, const ResidentPlan& pl) {
+  if (p.line_off == nullptr || pl.spread) return false;
+  const int rows = p.ny * p.nz;
+  int worst = 0;
+#pragma unroll 4
+  for (int r = 32 * threadIdx.x; r < rows; r += 32 * blockDim.x)
+    worst = max(worst, __ldg(p.line_off + min(rows, r + 32)) - __ldg(p.line_off + r));
+  return worst > pl.crowd;
+}
+
 // The y and z face lines of activated substrates take their face's values
 // (their ends, the x faces') in the x sweep's place: row number `at` of all
 // of them, by one warp, coalesced.
@@ -756,6 +771,7 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   const double* const coef =
       resident_coefs(p, pl, smem_raw, min(cta / ((p.ny * p.nz + 31) / 32), p.S - 1), min(cta / (xt * p.nz), p.S - 1),
                      min(cta / (xt * p.ny), p.S - 1));
+  const bool crowded = resident_crowded(p, pl);
   ResidentAgents<T> ag{};
   if (!pl.spread) ag = resident_agents<4>(p, w0, pl.agents, reinterpret_cast<double*>(keep));
   keep += static_cast<size_t>(pl.agents) * kAgentBytes;
@@ -768,11 +784,12 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   ResidentFace<T> face{};
   if (w0 < face_rows) face = resident_face(p, w0);
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
+  const bool spread = __syncthreads_or(crowded) || pl.spread;
+  if (spread) ag.a1 = ag.a0;
   const auto none = [] {};
   GridBarrier bar{barrier, gridDim.x};
   for (int step = 0; step < pl.nsteps; ++step) {
-    if (pl.spread) {
+    if (spread) {
       resident_spread(p, w0 * 32 + (threadIdx.x & 31), nw * 32);
       if (!bar.sync(p.status)) break;
     }
@@ -846,14 +863,15 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1)
   const int pitch = resident_pitch<T>(p.nx);
   const int xt = (p.nx + 31) / 32;
   const int face_rows = resident_face_rows(p, pl);
+  const bool crowded = resident_crowded(p, pl);
   const int ntx = (p.ny * p.nz + 31) / 32 * p.S, nty = xt * p.nz * p.S, ntz = xt * p.ny * p.S;
   asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
+  const bool spread = __syncthreads_or(crowded) || pl.spread;
   const auto none = [] {};
   GridBarrier bar{b.solve[m].barrier, static_cast<unsigned>(ctas)};
   for (int step = 0; step < b.nsteps; ++step) {
     for (int q = w0; q < face_rows; q += nw) resident_face_store(resident_face(p, q), p.nx);
-    if (pl.spread) {
+    if (spread) {
       resident_spread(p, (blockIdx.x - b.solve[m].cta0) * blockDim.x + threadIdx.x, ctas * blockDim.x);
       if (!bar.sync(p.status)) break;
     }
@@ -863,7 +881,7 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1)
       resident_tile<T, 0>(
           p, pl, coef, buf, l, [&] {
             resident_prefetch<T, 0>(p, tile + nw, ntx);
-            if (!pl.spread) ag = resident_agents<1>(p, tile, pl.agents, agents);
+            if (!spread) ag = resident_agents<1>(p, tile, pl.agents, agents);
           },
           [&] {
             if (ag.a1 > ag.a0) resident_sources(p, ag, buf, pitch, l.tile);
@@ -898,6 +916,26 @@ bool resident_spreads(const bfvm_ctx* c, const SweepParams<T>& p, long long roun
   const long long tiles = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
   const long long in_tiles = rounds * ((c->n_agents / tiles + 31) / 32);
   return in_tiles > 8 + 2 * ((static_cast<long long>(c->n_agents) * c->S + threads - 1) / threads);
+}
+
+// ResidentPlan::crowd: as many as no tile of agents spread evenly holds, and as
+// cost a tile of them more than the spread phase of `threads` threads.  us per
+// step, FP64, 10 steps, by averages alone -> with this (a launch per stage):
+//   50x50x50x2, 7,000 agents in a ball of 12 voxels' radius 29 -> 20 (32), 35,000
+//     156 -> 27 (34), 10,000 in one of 6 158 -> 27 (37), 2,000 in one of 2 189 ->
+//     32 (46), in eight voxels 279 -> 79 (87)
+//   100x100x100x2, 20,000 in a ball of 12 94 -> 34 (52); 128x128x128x1, 30,000 in
+//     one of 10 125 -> 37 (52); a plane of 300x260x3, 2,000 in a disc of 6 230 ->
+//     41 (55)
+// Slower than a launch per stage, which has more threads for them, where ten
+// agents and more lie in each voxel of a crowd: 70,000 in a ball of 12 43 (38),
+// 30,000 in a disc of 20 of the plane 81 (57).
+template <typename T>
+int resident_crowd(const bfvm_ctx* c, const SweepParams<T>& p, long long threads) {
+  if (p.line_off == nullptr || static_cast<long long>(c->n_agents) * c->S > INT_MAX / 2) return INT_MAX;
+  const long long tiles = (static_cast<long long>(c->ny) * c->nz + 31) / 32;
+  const long long each = (static_cast<long long>(c->n_agents) * c->S + threads - 1) / threads;
+  return static_cast<int>(std::max(2 * (c->n_agents / tiles) + 32, 32 * (4 + 2 * each)));
 }
 
 // Shapes and shared memory of a solve's run, with one tile per warp (many
@@ -1055,6 +1093,11 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
   if (resident_plan(c, p, nodes, two_d, false, sms, &pl, tiles, &smem)) {
     int grid = static_cast<int>(std::min<long long>(std::max(tiles[0], std::max(tiles[1], tiles[2])), sms));
     int threads = 32 * pl.warps;
+    // Eight warps an SM take that many agents' chains of divisions slower than a
+    // launch of their own: 50x50x50x2 FP64, us per step of this and of a launch
+    // per stage, 100,000 agents (11 a thread) 30 and 35, 200,000 (21) 48 and 38.
+    if (p.line_off != nullptr && static_cast<long long>(c->n_agents) * c->S > 12ll * sms * kSpreadThreads)
+      return BFVM_OK;
     if (pl.spread) {
       // Eight agents a thread, and two CTAs to an SM where their lines allow it:
       // a small grid leaves SMs to others' work (600x500x4 FP32 with 18,000
@@ -1063,11 +1106,14 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
           (static_cast<long long>(c->n_agents) * c->S + 8 * kSpreadThreads - 1) / (8 * kSpreadThreads);
       grid = static_cast<int>(std::max<long long>(grid, std::min<long long>(ctas, sms)));
       threads = std::max(threads, kSpreadThreads);
+    } else if (p.line_off != nullptr && static_cast<long long>(c->n_agents) * c->S > 4ll * grid * threads) {
+      threads = std::max(threads, kSpreadThreads);  // in case they crowd (resident_crowd)
     }
     // whether another such run finds room beside this one: 227 KB and eight warps an SM
     const long long per_sm = std::min<long long>(kSmemMax / smem, kResidentWarps / std::max(pl.warps, threads / 32));
     if (2 * grid > per_sm * sms && !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.5))
       return BFVM_OK;
+    pl.crowd = resident_crowd(c, p, static_cast<long long>(grid) * threads);
     int blocks = 0;
     BFVM_CUDA(persistent_grid(resident_kernel<T>, smem, grid, &blocks, threads));
     if (blocks < grid) return BFVM_OK;
@@ -1092,6 +1138,7 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
     pl.warps = warps;
     const long long all_x = static_cast<long long>(grid) * warps;
     pl.spread = resident_spreads(c, p, (tiles[0] + all_x - 1) / all_x, 32ll * grid * kManyWarps<T>) ? 1 : 0;
+    pl.crowd = resident_crowd(c, p, 32 * all_x);
     ResidentBatch<T, 1> b{};
     b.n = 1;
     b.solve[0] = {p, pl, 0, grid, barrier};
@@ -1186,6 +1233,7 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
           resident_spreads(members[m0 + m], b.solve[m].p, (tiles[m][0] + w - 1) / w, 32ll * warps * b.solve[m].ctas)
               ? 1
               : 0;
+      b.solve[m].pl.crowd = resident_crowd(members[m0 + m], b.solve[m].p, 32ll * warps * b.solve[m].ctas);
       cta += b.solve[m].ctas;
     }
     e = launch_many(b, grid, smem, warps, nsteps, st);
