@@ -414,7 +414,9 @@ int bfvm_get_sweep_schedule(bfvm_ctx* ctx, int* persistent);
  * sources and the pins are the same in both.  chain = 2: chain 1, except
  * that long y and z lines are solved by a partition
  * method (by default on lines of at least 512 voxels in FP64 and 448 in
- * FP32 and where it is the faster one): eight warps share each 32-line tile,
+ * FP32, of those below 576 in FP64 and of all in FP32 where the solve has too
+ * few lines for the serial sweep of two tiles per warp; the launch settings and
+ * the steps of a call do not enter): eight warps share each 32-line tile,
  * each warp running both recurrences over one eighth of the line, joined
  * through segment products that the host forms in extended precision at
  * set-up.  Its results are
@@ -427,7 +429,8 @@ int bfvm_get_sweep_schedule(bfvm_ctx* ctx, int* persistent);
 int bfvm_set_fp64_chain(bfvm_ctx* ctx, int chain);
 int bfvm_get_fp64_chain(bfvm_ctx* ctx, int* chain);
 /* The shortest y or z line that chain 2 solves partitioned: n_line >= 1,
- * or -1 for the default of the solve's precision (512 FP64, 448 FP32).
+ * or -1 for the default of the solve's precision (512 FP64, 448 FP32, and
+ * of these lines the ones that bfvm_set_fp64_chain says).
  * bfvm_get_partition_min_line returns the value in effect. */
 int bfvm_set_partition_min_line(bfvm_ctx* ctx, int n_line);
 int bfvm_get_partition_min_line(bfvm_ctx* ctx, int* n_line);

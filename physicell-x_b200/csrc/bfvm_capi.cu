@@ -77,6 +77,27 @@ void thomas_axis_host(int n, int S, const double* D, const double* decay, double
   }
 }
 
+static int part_min_line(const bfvm_ctx* c) {
+  return c->part_min_line >= 0 ? c->part_min_line : (c->eb == 8 ? kPartMinLine64 : kPartMinLine32);
+}
+
+template <typename T, int AXIS>
+bool partitioned(const bfvm_ctx* c, const SweepParams<T>& p) {
+  const int n = AXIS == 1 ? c->ny : c->nz;
+  if (c->fp64_chain != 2 || n < part_min_line(c) || (n + kRingRows - 1) / kRingRows > kPartMaxChunks ||
+      part_smem_bytes(c->eb, n) > 227 * 1024)
+    return false;
+  if (c->part_min_line >= 0 || (sizeof(T) == 8 && n >= kPartMinLinePair64)) return true;
+  SweepParams<T> whole = p;
+  whole.s_lo = 0;
+  whole.s_hi = c->S;
+  return !pair_takes<T, AXIS>(c->maps.pyz_w, whole, c->shape_cfg);
+}
+template bool partitioned<double, 1>(const bfvm_ctx*, const SweepParams<double>&);
+template bool partitioned<double, 2>(const bfvm_ctx*, const SweepParams<double>&);
+template bool partitioned<float, 1>(const bfvm_ctx*, const SweepParams<float>&);
+template bool partitioned<float, 2>(const bfvm_ctx*, const SweepParams<float>&);
+
 }  // namespace bfvm
 
 
@@ -87,17 +108,13 @@ constexpr int kStepEvents = 5;  // timing events per recorded step (enqueue_step
 // LOD steps per captured CUDA graph of bfvm_step (four launches each).
 constexpr int kGraphSteps = 16;
 
-int part_min_line(const bfvm_ctx* c) {
-  return c->part_min_line >= 0 ? c->part_min_line : (c->eb == 8 ? kPartMinLine64 : kPartMinLine32);
-}
-
 // Everything a captured step holds by value: the kernels' parameters are
 // built from these (device pointers change only with c->version), the
 // launch shapes from the sweep configuration.
 std::vector<long long> step_key(const bfvm_ctx* c, bool sources) {
   const SweepConfig& g = c->cfg;
   return {c->version, sources ? 1 : 0, c->n_agents, c->track, c->sub_streams, g.x_lines, g.yz_tile, g.yz_chunk, g.persistent,
-          g.fuse_sources, g.tmem, part_min_line(c), static_cast<long long>(reinterpret_cast<uintptr_t>(c->d_internal)),
+          g.fuse_sources, g.tmem, c->part_min_line, static_cast<long long>(reinterpret_cast<uintptr_t>(c->d_internal)),
           static_cast<long long>(reinterpret_cast<uintptr_t>(c->d_ae1))};
 }
 
@@ -105,19 +122,6 @@ void drop_step_graph(bfvm_ctx* c) {
   if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
   c->step_graph = nullptr;
   c->graph_key.clear();
-}
-
-// Whether the y (axis 1) or z (axis 2) sweep runs partitioned: chain 2, a
-// line of at least part_min_line voxels, and a tile that fits one CTA.
-// By default not where the sweep of two tiles per warp is the faster one.
-template <typename T, int AXIS>
-bool use_part(const bfvm_ctx* c, const SweepParams<T>& p) {
-  const int n = AXIS == 1 ? c->ny : c->nz;
-  if (c->fp64_chain != 2 || n < part_min_line(c) || (n + kRingRows - 1) / kRingRows > kPartMaxChunks ||
-      part_smem_bytes(c->eb, n) > 227 * 1024)
-    return false;
-  return c->part_min_line >= 0 || (sizeof(T) == 8 && n >= kPartMinLinePair64) ||
-         !pair_takes<T, AXIS>(c->maps.pyz_w, p, c->cfg);
 }
 
 // The launches of one LOD step on c->stream (also while capturing): the
@@ -137,12 +141,12 @@ int enqueue_step(bfvm_ctx* c, const SweepParams<T>& p, bool standalone, cudaEven
   if (ev) BFVM_CUDA(cudaEventRecord(ev[1], st));
   BFVM_CUDA(launch_sweep_x<T>(c->maps, p, c->cfg, st));
   if (ev) BFVM_CUDA(cudaEventRecord(ev[2], st));
-  if (use_part<T, 1>(c, p))
+  if (partitioned<T, 1>(c, p))
     BFVM_CUDA((launch_part<T, 1>(c->maps.ry, p, c->part[1], st)));
   else
     BFVM_CUDA(launch_sweep_y<T>(c->maps, p, c->cfg, st));
   if (ev) BFVM_CUDA(cudaEventRecord(ev[3], st));
-  if (use_part<T, 2>(c, p))
+  if (partitioned<T, 2>(c, p))
     BFVM_CUDA((launch_part<T, 2>(c->maps.rz, p, c->part[2], st)));
   else
     BFVM_CUDA(launch_sweep_z<T>(c->maps, p, c->cfg, st));
@@ -647,6 +651,7 @@ int bfvm_create(const bfvm_config* cfg, bfvm_ctx** out) {
     delete c;
     return BFVM_ERR_SHAPE;
   }
+  c->shape_cfg = c->cfg;
   auto fail = [&](int rc) {
     bfvm_destroy(c);
     return rc;

@@ -52,6 +52,7 @@ struct bfvm_ctx {
   double* d_sums = nullptr;    // partial sums + result
   bfvm::FieldMaps maps{};
   bfvm::SweepConfig cfg{};
+  bfvm::SweepConfig shape_cfg{};  // what cfg was at first, by the shape
   // agents
   int n_agents = 0, cap_agents = 0;
   int* d_voxel = nullptr;
@@ -205,6 +206,14 @@ struct NodeLines {
   const int* order[2];
   int most[2];  // nodes of 32 lines (32 q ..) at most
 };
+// bfvm_capi.cu: whether the y (axis 1) or z (axis 2) sweep of a step runs
+// partitioned: chain 2, a line of at least part_min_line voxels, and a tile that
+// fits one CTA; by default not where the sweep of two tiles per warp is the
+// faster one.  The partition has bits of its own, so what decides is the solve's
+// alone: not the launch settings, nor the substrates or steps of a launch.
+template <typename T, int AXIS>
+bool partitioned(const bfvm_ctx* c, const SweepParams<T>& p);
+
 // bfvm_resident.cu: nsteps whole steps of a small grid in one launch on st,
 // sources (p.line_off) and 2-D nodes included; *launched false where the solve
 // is too large for it or a launch setting asks for another form.

@@ -947,6 +947,7 @@ bool resident_plan(const bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& 
   if (c->timing || (p.line_off != nullptr && c->track) || c->sub_streams != 1 || g.persistent != 1 || g.tmem != 1 ||
       g.x_lines != 32 || g.yz_tile != 32)
     return false;
+  if (!two_d && (partitioned<T, 1>(c, p) || partitioned<T, 2>(c, p))) return false;  // (serial lines here)
   const int n[3] = {c->nx, c->ny, c->nz}, S = c->S;
   const int naxes = two_d ? 2 : 3;
   ResidentPlan pl{};
