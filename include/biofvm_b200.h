@@ -399,7 +399,9 @@ int bfvm_set_substrate_streams(bfvm_ctx* ctx, int streams);
 int bfvm_get_substrate_streams(const bfvm_ctx* ctx, int* streams);
 /* Where bfvm_step applies the agents: fused = 0 (default) the standalone
  * source kernel ahead of the sweeps, 1 inside the x sweep, on the staged
- * tile.  Both give the same bits. */
+ * tile.  Both give the same bits.  Both are forms of a launch per stage: a
+ * solve for which this was called, with either value, takes no several steps
+ * per launch (bfvm_step). */
 int bfvm_set_fused_sources(bfvm_ctx* ctx, int fused);
 int bfvm_get_sweep_schedule(bfvm_ctx* ctx, int* persistent);
 /* Arithmetic of the FP64 forward elimination.  chain = 0 (default): the
@@ -454,8 +456,8 @@ int bfvm_set_sweep_tmem(bfvm_ctx* ctx, int on);
 int bfvm_tmem_sweep_plan(int axis, int n_line, int tmem_level, int* smem_rings, int* tmem_rings, int* input_slots);
 
 /* Number of this library's kernels launched by the calls so far (counted on
- * the host at each launch; a launch that runs whole steps of a small grid
- * counts once for every stage of theirs that it stands for). */
+ * the host at each launch and at each replay of a graph; a launch that runs
+ * several steps is one). */
 long long bfvm_kernel_launches(void);
 
 /* Per-kernel timing, the device counterpart of the reference's per-step
@@ -514,7 +516,8 @@ int bfvm_batch_get_schedule(bfvm_batch* batch, int* mode, int* yz_chunk, int* or
                             int* graph_steps);
 /* Mode 2: members of at least `values` voxel-substrate values (nx*ny*nz*S,
  * default 2097152 = 128^3 x 1) that do not run side by side with others are
- * stepped with their own kernels. */
+ * stepped with their own kernels.  Setting it asks for these two forms: no
+ * member of a batch for which it was set runs side by side with others. */
 int bfvm_batch_set_direct_threshold(bfvm_batch* batch, long long values);
 int bfvm_batch_get_direct_threshold(bfvm_batch* batch, long long* values);
 /* Time trial_steps fused steps under each candidate schedule, keep the

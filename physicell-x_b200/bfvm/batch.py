@@ -67,7 +67,8 @@ class Batch:
 
     def set_direct_threshold(self, values):
         """Mode 2: members of at least `values` voxel-substrate values that do
-        not run side by side with others step with their own kernels."""
+        not run side by side with others step with their own kernels;
+        setting it, no member runs side by side with others."""
         check(self.L.bfvm_batch_set_direct_threshold(self.h, C.c_longlong(int(values))),
               "bfvm_batch_set_direct_threshold")
 

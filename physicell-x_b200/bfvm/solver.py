@@ -347,7 +347,8 @@ class Microenvironment:
 
     def set_fused_sources(self, fused=True):
         """Apply the agents inside the x sweep (True) or with the standalone
-        source kernel ahead of the sweeps (False, the default)."""
+        source kernel ahead of the sweeps (False, the default).  Either asks
+        for a launch per stage: such a solve runs no several steps per launch."""
         check(self.L.bfvm_set_fused_sources(self.h, 1 if fused else 0), "bfvm_set_fused_sources")
 
     def set_substrate_streams(self, streams=1):

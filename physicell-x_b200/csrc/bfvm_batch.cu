@@ -36,12 +36,11 @@ struct bfvm_batch {
                         // 2: the members that bfvm_resident.cu takes side by side in one launch; of the
                         // others, as 1 those under direct_min values, the rest with their own kernels
                         // (enqueue_step_on) on the batch stream
+  bool direct_set = false;         // bfvm_batch_set_direct_threshold was called: its two forms are asked for
   long long direct_min = 2097152;  // mode 2: N*S (voxel-substrate values) from which a member steps directly
   std::vector<bfvm_ctx*> direct;  // mode 2: the members stepped directly (set with the tables)
   std::vector<bfvm_ctx*> resident;  // mode 2: the members that run side by side in one launch, of either kind
-  bool batched = false;             // there are members under direct_min
-  int direct_launches = 0;        // the kernels per step of the members from direct_min on
-  int resident_launches = 0;      // those of them that stand for stages of the one launch
+  int direct_launches = 0;        // the direct members' kernels per step
   // mode 2: the direct members run on up to kSideStreams side streams, forked
   // from the batch stream and joined back around each run of steps, so that
   // the members' own persistent kernels share the GPU; direct_lane[i] is the
@@ -71,6 +70,7 @@ struct bfvm_batch {
   size_t g_smem = 0;
   int g_grid = 0, g_cap = 0, g_steps = 0, g_mode = -1;
   int g_items[3] = {0, 0, 0};
+  int g_resident = 0;  // its launches of the members that run side by side
   long long launches = 0;
   std::vector<int> env_of;  // member index -> position in the device tables
   bfvm_ctx* stall = nullptr;  // bfvm_batch_inject_stall: member whose next step's x tiles never count
@@ -126,9 +126,7 @@ int build_tables(bfvm_batch* b, bool sources) {
   std::vector<int> idx;
   b->direct.clear();
   b->resident.clear();
-  b->batched = false;
   b->direct_launches = 0;
-  b->resident_launches = 0;
   // Dense agents cost the one launch more than a launch per stage, whose
   // threads all take them: 10 FP64 members of edges to 55 with agents in 1 voxel
   // of 6, six steps, 466 -> 378 us a call alone, but 247 -> 308 for each of three
@@ -141,18 +139,13 @@ int build_tables(bfvm_batch* b, bool sources) {
   const bool sparse = !sources || 32 * agents <= voxels;
   for (int q = 0; q < n; ++q) {
     bfvm_ctx* c = b->members[q];
-    const bool direct = b->mode == 2 && 1LL * c->nx * c->ny * c->nz * c->S >= b->direct_min;
-    const bool resident = b->mode == 2 && sparse && resident_member<T>(c, sources);
-    if (resident) b->resident.push_back(c);
-    if (resident && !direct) b->batched = true;
-    if (direct) {
-      if (!resident) b->direct.push_back(c);
-      const int launches = 3 + ((sources && c->n_agents > 0 && !c->cfg.fuse_sources) ? 1 : 0);
-      b->direct_launches += launches;
-      if (resident) b->resident_launches += launches;
-    } else if (!resident) {
+    if (b->mode == 2 && sparse && !b->direct_set && resident_member<T>(c, sources)) {
+      b->resident.push_back(c);
+    } else if (b->mode == 2 && 1LL * c->nx * c->ny * c->nz * c->S >= b->direct_min) {
+      b->direct.push_back(c);
+      b->direct_launches += 3 + ((sources && c->n_agents > 0 && !c->cfg.fuse_sources) ? 1 : 0);
+    } else {
       idx.push_back(q);
-      b->batched = true;
     }
   }
   // the direct members' side streams: the largest member first onto the
@@ -286,8 +279,10 @@ cudaError_t enqueue_fused_step(bfvm_batch* b, int stall_env) {
 // stall_env >= 0 (fault injection, fused schedule only): that table entry's
 // finished-x-tile counter starts far below zero, so its y tiles wait on x
 // tiles that never count up and their bounded waits run out.
+// *resident receives the launches of the members that run side by side.
 template <typename T>
-cudaError_t enqueue_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
+cudaError_t enqueue_steps(bfvm_batch* b, int nsteps, int* resident, int stall_env = -1) {
+  *resident = 0;
   if (b->mode >= 1) {
     const int K = std::min(static_cast<int>(b->direct.size()), static_cast<int>(b->side.size()));
     cudaError_t e = cudaSuccess;
@@ -298,7 +293,7 @@ cudaError_t enqueue_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
     }
     if (e == cudaSuccess && !b->resident.empty())
       e = run_resident_members<T>(b->resident.data(), static_cast<int>(b->resident.size()), b->built_sources, nsteps,
-                                  b->stream);
+                                  b->stream, resident);
     for (int s = 0; s < nsteps && e == cudaSuccess; ++s)
       e = launch_batch_sweeps<T>(b->d_hdr, static_cast<const BatchEnv<T>*>(b->d_envs), b->d_pre, b->cap, b->items,
                                  b->axis_smem, b->stream);
@@ -321,18 +316,18 @@ cudaError_t enqueue_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
 }
 
 // The batched kernels of one step (the directly stepped members count their
-// own launches as they enqueue them).  The launch that runs the resident
-// members' steps counts as the stages it stands for.
+// own launches as they enqueue them).
 int kernels_per_step(const bfvm_batch* b) {
   if (b->mode == 0) return 1;
-  return b->mode == 1 || b->batched ? 3 : 0;
+  return (b->items[0] > 0) + (b->items[1] > 0) + (b->items[2] > 0);
 }
 
 template <typename T>
 int launch_steps(bfvm_batch* b, int nsteps, int stall_env = -1) {
-  BFVM_CUDA(enqueue_steps<T>(b, nsteps, stall_env));
-  note_launches(nsteps * (kernels_per_step(b) + b->resident_launches));
-  b->launches += nsteps * (kernels_per_step(b) + b->direct_launches);
+  int resident = 0;
+  BFVM_CUDA(enqueue_steps<T>(b, nsteps, &resident, stall_env));
+  note_launches(nsteps * kernels_per_step(b) + resident);
+  b->launches += nsteps * (kernels_per_step(b) + b->direct_launches) + resident;
   return BFVM_OK;
 }
 
@@ -343,7 +338,7 @@ int capture_graph(bfvm_batch* b) {
   BFVM_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   set_launch_capture(true);  // the replays count the launches
   {
-    const cudaError_t e2 = enqueue_steps<T>(b, b->graph_steps);
+    const cudaError_t e2 = enqueue_steps<T>(b, b->graph_steps, &b->g_resident);
     if (e2 != cudaSuccess) {
       set_launch_capture(false);
       cudaStreamEndCapture(b->stream, &g);
@@ -427,8 +422,9 @@ int step_impl(bfvm_batch* b, int nsteps, bool sources) {
     }
     while (left >= b->g_steps) {
       BFVM_CUDA(cudaGraphLaunch(b->gexec, b->stream));
-      note_launches(b->g_steps * (kernels_per_step(b) + b->direct_launches));
-      b->launches += b->g_steps * (kernels_per_step(b) + b->direct_launches);
+      const int launches = b->g_steps * (kernels_per_step(b) + b->direct_launches) + b->g_resident;
+      note_launches(launches);
+      b->launches += launches;
       left -= b->g_steps;
     }
   }
@@ -568,8 +564,9 @@ int bfvm_batch_set_schedule(bfvm_batch* b, int mode, int yz_chunk, int order, in
 
 int bfvm_batch_set_direct_threshold(bfvm_batch* b, long long values) {
   if (!b || values < 1) return BFVM_ERR_ARG;
-  if (values != b->direct_min) {
+  if (values != b->direct_min || !b->direct_set) {
     b->direct_min = values;
+    b->direct_set = true;
     b->dirty = true;
     drop_graph(b);
   }

@@ -229,14 +229,11 @@ int run_steps_plain(bfvm_ctx* c, int nsteps, bool sources) {
   const bool standalone = sources && c->n_agents > 0 && !c->cfg.fuse_sources;
   const SweepParams<T> p = make_params<T>(c, sources && !standalone);
   {
-    // a small grid: the whole run in one launch, each stage counted as one
-    bool launched = false;
-    const int rc = run_resident<T>(c, make_params<T>(c, sources), NodeLines{}, false, nsteps, c->stream, &launched);
-    if (rc != BFVM_OK) return rc;
-    if (launched) {
-      note_launches(nsteps * (3 + (standalone ? 1 : 0)));
-      return BFVM_OK;
-    }
+    // a small grid: the whole run in one launch
+    int launches = 0;
+    const int rc = run_resident<T>(c, make_params<T>(c, sources), NodeLines{}, false, nsteps, c->stream, &launches);
+    note_launches(launches);
+    if (rc != BFVM_OK || launches > 0) return rc;
   }
   // Runs of steps replay a captured graph of kGraphSteps steps (the same
   // launches, so the same bits), which removes most of the per-launch host
@@ -1382,6 +1379,7 @@ extern "C" int bfvm_set_fused_sources(bfvm_ctx* c, int fused) {
   DeviceGuard g(c->device);
   BFVM_CUDA(cudaStreamSynchronize(c->stream));
   change_setting(c, &c->cfg.fuse_sources, fused);
+  change_setting(c, &c->sources_set, true);
   return BFVM_OK;
 }
 

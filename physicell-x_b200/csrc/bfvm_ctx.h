@@ -110,6 +110,7 @@ struct bfvm_ctx {
   cudaGraphExec_t step_graph = nullptr;
   std::vector<long long> graph_key;
   // per-kernel timing: 4 events per recorded step
+  bool sources_set = false;    // bfvm_set_fused_sources was called: its form, a launch per stage, is asked for
   bool timing = false;
   int timed_steps = 0;
   std::vector<cudaEvent_t> events;
@@ -215,17 +216,19 @@ template <typename T, int AXIS>
 bool partitioned(const bfvm_ctx* c, const SweepParams<T>& p);
 
 // bfvm_resident.cu: nsteps whole steps of a small grid in one launch on st,
-// sources (p.line_off) and 2-D nodes included; *launched false where the solve
-// is too large for it or a launch setting asks for another form.
+// sources (p.line_off) and 2-D nodes included; *launches is 0 where the solve is
+// too large for it or a launch setting asks for another form.
 template <typename T>
 int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, int nsteps, cudaStream_t st,
-                 bool* launched);
+                 int* launches);
 // Whether a batch's member may run beside others in run_resident_members, and
-// nsteps whole steps of such members on st.
+// nsteps whole steps of such members on st, in as many launches as are added to
+// *launches.
 template <typename T>
 bool resident_member(bfvm_ctx* c, bool sources);
 template <typename T>
-cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sources, int nsteps, cudaStream_t st);
+cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sources, int nsteps, cudaStream_t st,
+                                 int* launches);
 cudaError_t resident_set_wait_limit(unsigned long long ns);
 
 inline AgentTrack track_params(const bfvm_ctx* c) {

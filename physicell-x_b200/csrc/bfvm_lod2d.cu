@@ -188,16 +188,13 @@ NodeLines node_lines(const bfvm_ctx* c) {
 template <typename T>
 int run_steps_2d(bfvm_ctx* c, int nsteps, bool sources) {
   {
-    // a small grid: the whole run in one launch, each stage counted as one
+    // a small grid: the whole run in one launch
     const bool src = sources && c->n_agents > 0;
     SweepParams<T> p = make_params_2d<T>(c, src);
-    bool launched = false;
-    const int rc = run_resident<T>(c, p, node_lines(c), true, nsteps, c->stream, &launched);
-    if (rc != BFVM_OK) return rc;
-    if (launched) {
-      note_launches(nsteps * (2 + (src ? 1 : 0) + (c->n_nodes > 0 ? 3 : 0)));
-      return BFVM_OK;
-    }
+    int launches = 0;
+    const int rc = run_resident<T>(c, p, node_lines(c), true, nsteps, c->stream, &launches);
+    note_launches(launches);
+    if (rc != BFVM_OK || launches > 0) return rc;
   }
   const SweepParams<T> p = make_params_2d<T>(c, false);
   for (int st = 0; st < nsteps; ++st) {

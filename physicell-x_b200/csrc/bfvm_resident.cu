@@ -944,7 +944,7 @@ template <typename T>
 bool resident_plan(const bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, bool many, int sms,
                    ResidentPlan* plan, long long* tiles, size_t* smem) {
   const SweepConfig& g = c->cfg;
-  if (c->timing || (p.line_off != nullptr && c->track) || c->sub_streams != 1 || g.persistent != 1 || g.tmem != 1 ||
+  if (c->timing || c->sources_set || (p.line_off != nullptr && c->track) || c->sub_streams != 1 || g.persistent != 1 || g.tmem != 1 ||
       g.x_lines != 32 || g.yz_tile != 32)
     return false;
   if (!two_d && (partitioned<T, 1>(c, p) || partitioned<T, 2>(c, p))) return false;  // (serial lines here)
@@ -1004,7 +1004,8 @@ bool resident_plan(const bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& 
 }
 
 template <typename T, int N>
-cudaError_t launch_many(ResidentBatch<T, N>& b, int grid, size_t smem, int warps, int nsteps, cudaStream_t st) {
+cudaError_t launch_many(ResidentBatch<T, N>& b, int grid, size_t smem, int warps, int nsteps, cudaStream_t st,
+                        int* launches) {
   int blocks = 0;
   cudaError_t e = persistent_grid(resident_many_kernel<T, N>, smem, grid, &blocks, 32 * warps);
   if (e != cudaSuccess) return e;
@@ -1014,6 +1015,7 @@ cudaError_t launch_many(ResidentBatch<T, N>& b, int grid, size_t smem, int warps
     void* args[] = {&b};
     e = cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(resident_many_kernel<T, N>), dim3(grid),
                                     dim3(32 * warps), args, smem, st);
+    if (e == cudaSuccess) ++*launches;
   }
   return e;
 }
@@ -1081,8 +1083,8 @@ int sm_count(int device, int* sms) {
 
 template <typename T>
 int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, int nsteps, cudaStream_t st,
-                 bool* launched) {
-  *launched = false;
+                 int* launches) {
+  *launches = 0;
   if (nsteps < 1) return BFVM_OK;
   int sms = 0;
   const int rc = sm_count(c->device, &sms);
@@ -1123,8 +1125,8 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
       void* args[] = {const_cast<SweepParams<T>*>(&p), &pl, const_cast<NodeLines*>(&nodes), &barrier};
       BFVM_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(resident_kernel<T>), dim3(grid),
                                             dim3(threads), args, smem, st));
+      ++*launches;
     }
-    *launched = true;
     return BFVM_OK;
   }
   if (!two_d && resident_plan(c, p, nodes, false, true, sms, &pl, tiles, &smem)) {
@@ -1143,8 +1145,7 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
     ResidentBatch<T, 1> b{};
     b.n = 1;
     b.solve[0] = {p, pl, 0, grid, barrier};
-    BFVM_CUDA(launch_many(b, grid, smem, pl.spread ? kManyWarps<T> : warps, nsteps, st));
-    *launched = true;
+    BFVM_CUDA(launch_many(b, grid, smem, pl.spread ? kManyWarps<T> : warps, nsteps, st, launches));
   }
   return BFVM_OK;
 }
@@ -1163,7 +1164,8 @@ bool resident_member(bfvm_ctx* c, bool sources) {
 }
 
 template <typename T>
-cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sources, int nsteps, cudaStream_t st) {
+cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sources, int nsteps, cudaStream_t st,
+                                 int* launches) {
   ResidentBatch<T, kResidentMembers> b{};
   int sms = 0;
   if (count == 0 || sm_count(members[0]->device, &sms) != BFVM_OK) return cudaGetLastError();
@@ -1237,7 +1239,7 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
       b.solve[m].pl.crowd = resident_crowd(members[m0 + m], b.solve[m].p, 32ll * warps * b.solve[m].ctas);
       cta += b.solve[m].ctas;
     }
-    e = launch_many(b, grid, smem, warps, nsteps, st);
+    e = launch_many(b, grid, smem, warps, nsteps, st, launches);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -1245,12 +1247,12 @@ cudaError_t run_resident_members(bfvm_ctx* const* members, int count, bool sourc
 
 template bool resident_member<double>(bfvm_ctx*, bool);
 template bool resident_member<float>(bfvm_ctx*, bool);
-template cudaError_t run_resident_members<double>(bfvm_ctx* const*, int, bool, int, cudaStream_t);
-template cudaError_t run_resident_members<float>(bfvm_ctx* const*, int, bool, int, cudaStream_t);
+template cudaError_t run_resident_members<double>(bfvm_ctx* const*, int, bool, int, cudaStream_t, int*);
+template cudaError_t run_resident_members<float>(bfvm_ctx* const*, int, bool, int, cudaStream_t, int*);
 template int run_resident<double>(bfvm_ctx*, const SweepParams<double>&, const NodeLines&, bool, int, cudaStream_t,
-                                  bool*);
+                                  int*);
 template int run_resident<float>(bfvm_ctx*, const SweepParams<float>&, const NodeLines&, bool, int, cudaStream_t,
-                                 bool*);
+                                 int*);
 
 cudaError_t resident_set_wait_limit(unsigned long long ns) { return set_module_wait_limit(ns); }
 
