@@ -445,8 +445,9 @@ int bfvm_get_partition_min_line(bfvm_ctx* ctx, int* n_line);
  * the shared-memory rings; 2 also in the FP64 x sweep on lines of 17 to 32;
  * 0 shared memory alone.  Every level gives the same bits. */
 int bfvm_set_sweep_tmem(bfvm_ctx* ctx, int on);
-/* The tensor-memory sweep a persistent sweep would run on lines of n_line
- * voxels (host arithmetic, no device needed): axis 0 = the FP64 x sweep
+/* The single-tile tensor-memory sweep's plan for lines of n_line voxels (host
+ * arithmetic, no device needed).  Where a solve has tiles enough, the sweep of
+ * two tiles per warp, with rings of its own, runs in its place.  axis 0 = the FP64 x sweep
  * (agents not fused into it), 1 = the FP64 y or z sweep, 2 = the FP32 y or
  * z sweep, 3 = the FP32 x sweep; tmem_level as
  * bfvm_set_sweep_tmem.  Sets the shared-memory rings, TMEM rings and input
