@@ -560,14 +560,34 @@ __device__ __forceinline__ void resident_spread(const SweepParams<T>& p, unsigne
   }
 }
 
+// What a launch looks up for the two below, read before the rest of its set-up,
+// which hides the latency.
+struct ResidentLook {
+  int from, to;  // this thread's first x tile in the sorted agents
+  int on;        // activation of substrate `lane`
+};
+
+template <typename T>
+__device__ __forceinline__ ResidentLook resident_look(const SweepParams<T>& p, const ResidentPlan& pl) {
+  ResidentLook l{};
+  const int rows = p.ny * p.nz, r = 32 * threadIdx.x, s = threadIdx.x & 31;
+  if (p.line_off != nullptr && !pl.spread && r < rows) {
+    l.from = __ldg(p.line_off + r);
+    l.to = __ldg(p.line_off + min(rows, r + 32));
+  }
+  if (s < p.S) l.on = __ldg(p.active + s);
+  return l;
+}
+
 // The face lines of all activated substrates.  How many are activated is read
 // when the launch runs: a captured launch outlives the activation it was
 // captured under, and the lines it leaves out of the sweeps follow the device's.
 template <typename T>
-__device__ __forceinline__ int resident_face_rows(const SweepParams<T>& p, const ResidentPlan& pl) {
+__device__ __forceinline__ int resident_face_rows(const SweepParams<T>& p, const ResidentPlan& pl,
+                                                  const ResidentLook& l) {
   if (pl.face_rows == 0) return 0;
-  int on = 0;
-  for (int s0 = 0; s0 < p.S; s0 += 32) {
+  int on = __popc(__ballot_sync(0xffffffffu, l.on != 0));
+  for (int s0 = 32; s0 < p.S; s0 += 32) {
     const int s = s0 + (threadIdx.x & 31);
     on += __popc(__ballot_sync(0xffffffffu, s < p.S && p.active[s] != 0));
   }
@@ -578,12 +598,12 @@ __device__ __forceinline__ int resident_face_rows(const SweepParams<T>& p, const
 // (the threads of a CTA look at all of them between them, so every CTA of the
 // run comes to the same answer).
 template <typename T>
-__device__ __forceinline__ bool resident_crowded(const SweepParams<T>& p, const ResidentPlan& pl) {
+__device__ __forceinline__ bool resident_crowded(const SweepParams<T>& p, const ResidentPlan& pl,
+                                                 const ResidentLook& l) {
   if (p.line_off == nullptr || pl.spread) return false;
   const int rows = p.ny * p.nz;
-  int worst = 0;
-#pragma unroll 4
-  for (int r = 32 * threadIdx.x; r < rows; r += 32 * blockDim.x)
+  int worst = l.to - l.from;
+  for (int r = 32 * (threadIdx.x + blockDim.x); r < rows; r += 32 * blockDim.x)
     worst = max(worst, __ldg(p.line_off + min(rows, r + 32)) - __ldg(p.line_off + r));
   return worst > pl.crowd;
 }
@@ -756,6 +776,7 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
     resident_kernel(const SweepParams<T> p, const ResidentPlan pl, const NodeLines nd, unsigned long long* barrier) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int warp = threadIdx.x >> 5;
+  const ResidentLook look = resident_look(p, pl);
   // Neighbouring tiles on different SMs.  (Warps past the plan's, there for the
   // sources, find no tile.)
   const int w0 = blockIdx.x + gridDim.x * warp, nw = gridDim.x * (blockDim.x >> 5);
@@ -771,7 +792,6 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   const double* const coef =
       resident_coefs(p, pl, smem_raw, min(cta / ((p.ny * p.nz + 31) / 32), p.S - 1), min(cta / (xt * p.nz), p.S - 1),
                      min(cta / (xt * p.ny), p.S - 1));
-  const bool crowded = resident_crowded(p, pl);
   ResidentAgents<T> ag{};
   if (!pl.spread) ag = resident_agents<4>(p, w0, pl.agents, reinterpret_cast<double*>(keep));
   keep += static_cast<size_t>(pl.agents) * kAgentBytes;
@@ -780,7 +800,8 @@ __global__ void __launch_bounds__(32 * kResidentWarps, 1)
   const ResidentNodes<T> yn = resident_nodes(p, nd, 1, w0, pl.nodes[1], keep);
   const int l0 = w0 % ((p.ny + 31) / 32) * 32;  // (of a plane)
   __syncwarp();
-  const int face_rows = resident_face_rows(p, pl);
+  const bool crowded = resident_crowded(p, pl, look);
+  const int face_rows = resident_face_rows(p, pl, look);
   ResidentFace<T> face{};
   if (w0 < face_rows) face = resident_face(p, w0);
   asm volatile("cp.async.wait_all;" ::: "memory");
@@ -851,6 +872,7 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1)
   const SweepParams<T>& p = b.solve[m].p;
   const ResidentPlan& pl = b.solve[m].pl;
   const int ctas = b.solve[m].ctas;
+  const ResidentLook look = resident_look(p, pl);
   const double* const coef = resident_coefs(p, pl, smem_raw, 0, 0, 0);
   const int warp = threadIdx.x >> 5;
   const int nw = ctas * pl.warps;
@@ -862,8 +884,8 @@ __global__ void __launch_bounds__(32 * kManyWarps<T>, 1)
       reinterpret_cast<double*>(keep + static_cast<size_t>(32) * resident_pitch<T>(pl.line) * sizeof(T));
   const int pitch = resident_pitch<T>(p.nx);
   const int xt = (p.nx + 31) / 32;
-  const int face_rows = resident_face_rows(p, pl);
-  const bool crowded = resident_crowded(p, pl);
+  const int face_rows = resident_face_rows(p, pl, look);
+  const bool crowded = resident_crowded(p, pl, look);
   const int ntx = (p.ny * p.nz + 31) / 32 * p.S, nty = xt * p.nz * p.S, ntz = xt * p.ny * p.S;
   asm volatile("cp.async.wait_all;" ::: "memory");
   const bool spread = __syncthreads_or(crowded) || pl.spread;
