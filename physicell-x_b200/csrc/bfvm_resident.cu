@@ -31,8 +31,8 @@
 // With one tile per warp it won at every size it takes, up to what an SM holds:
 // eight warps of 254 registers, or 227 KB of line buffers and coefficients.
 // With several, the next tile's lines prefetched to the L2: see resident_wins;
-// 24 uneven solves of edges 24 to 128: FP32 (247 MB) 594 -> 429 us a step, FP64
-// 932 -> 702.  Where it gives way to a launch per stage: resident_shares.
+// 24 uneven solves of edges 24 to 128: FP32 (247 MB) 580 -> 411 us a step, FP64
+// 912 -> 673.  Where it gives way to a launch per stage: resident_shares.
 #include <algorithm>
 #include <climits>
 #include <cmath>
