@@ -547,15 +547,50 @@ __device__ __forceinline__ void resident_spread(const SweepParams<T>& p, unsigne
       rho[u] = p.f + (static_cast<size_t>(s) * rows + row) * p.nxp + i;
       x[u] = __ldcg(rho[u]);
     }
+    // The first agent of each run; then what the runs go on to, where agents are
+    // stacked, one by one: a lane's first run, then its second.  (Stacks leave
+    // most of a warp's agents without a run of their own: taking the runs by the
+    // agents' places, a warp waited four times for the longest of its lanes:
+    // 50x50x50x2 FP64, 70,000 agents in a ball of 12 voxels 43 -> 37 us a step, a
+    // plane of 300x260x3, 10,000 in a disc of 20 54 -> 48, 30,000 81 -> 67.)
+    double r[kAgents];
+    unsigned more = 0;
 #pragma unroll
     for (int u = 0; u < kAgents; ++u) {
       if (rho[u] == nullptr) continue;
       const unsigned e = e0 + u * threads;
       const int s = static_cast<int>(e / n), q = static_cast<int>(e - s * n);
+      const double off = sizeof(T) == 4 ? p.off[s] : 0.0;
+      r[u] = static_cast<double>(x[u]);
+      if constexpr (kF32<T>) r[u] += off;
+      r[u] = agent_update(r[u], k1[u], k2[u], k3[u], q, s, p.track);
+      if (q + 1 < n && after[u] == key[u]) {
+        more |= 1u << u;
+      } else {
+        if constexpr (kF32<T>) r[u] -= off;
+        *rho[u] = static_cast<T>(r[u]);
+      }
+    }
+    while (more != 0) {
+      const int pick = __ffs(more) - 1;
+      more &= more - 1;
+      T* at = rho[0];
+      double v = r[0];
+      unsigned mine = key[0];
+#pragma unroll
+      for (int u = 1; u < kAgents; ++u) {
+        if (pick != u) continue;
+        at = rho[u];
+        v = r[u];
+        mine = key[u];
+      }
+      const unsigned e = e0 + pick * threads;
+      const int s = static_cast<int>(e / n);
       const size_t sn = static_cast<size_t>(s) * p.n_sorted;
-      apply_run<T>(&x[u], q, key[u], k1[u], k2[u], k3[u], q + 1 < n && after[u] == key[u] ? n : q + 1, p.a_key,
-                   p.ac1 + sn, p.ac2 + sn, p.ae2 + sn, sizeof(T) == 4 ? p.off[s] : 0.0, s, p.track);
-      *rho[u] = x[u];
+      for (int q = static_cast<int>(e - s * n) + 1; q < n && __ldg(p.a_key + q) == mine; ++q)
+        v = agent_update(v, __ldg(p.ac1 + sn + q), __ldg(p.ac2 + sn + q), __ldg(p.ae2 + sn + q), q, s, p.track);
+      if constexpr (kF32<T>) v -= p.off[s];
+      *at = static_cast<T>(v);
     }
   }
 }
@@ -944,14 +979,14 @@ bool resident_spreads(const bfvm_ctx* c, const SweepParams<T>& p, long long roun
 // cost a tile of them more than the spread phase of `threads` threads.  us per
 // step, FP64, 10 steps, by averages alone -> with this (a launch per stage):
 //   50x50x50x2, 7,000 agents in a ball of 12 voxels' radius 29 -> 20 (32), 35,000
-//     156 -> 27 (34), 10,000 in one of 6 158 -> 27 (37), 2,000 in one of 2 189 ->
+//     156 -> 27 (34), 10,000 in one of 6 158 -> 25 (37), 2,000 in one of 2 189 ->
 //     32 (46), in eight voxels 279 -> 79 (87)
 //   100x100x100x2, 20,000 in a ball of 12 94 -> 34 (52); 128x128x128x1, 30,000 in
 //     one of 10 125 -> 37 (52); a plane of 300x260x3, 2,000 in a disc of 6 230 ->
-//     41 (55)
-// Slower than a launch per stage, which has more threads for them, where ten
-// agents and more lie in each voxel of a crowd: 70,000 in a ball of 12 43 (38),
-// 30,000 in a disc of 20 of the plane 81 (57).
+//     39 (55)
+// Slower than a launch per stage, which has more threads for them, where stacks
+// are deep over a whole crowd: 30,000 in a disc of 20 of the plane (24 a voxel)
+// 67 (57), FP32 65 (52); 64x64x64x2 FP32, 100,000 in a ball of 24 41 (37).
 template <typename T>
 int resident_crowd(const bfvm_ctx* c, const SweepParams<T>& p, long long threads) {
   if (p.line_off == nullptr || static_cast<long long>(c->n_agents) * c->S > INT_MAX / 2) return INT_MAX;
