@@ -152,9 +152,10 @@ int bfvm_agent_constants_device(int n, int S, double dt, double voxel_volume, co
  *  diffusion_decay_solver__constant_coefficients_LOD_3D_BLOCKING]
  * (BioFVM_microenvironment.cpp:1370-1384; BioFVM_solvers.cpp:102-780):
  * Dirichlet pin, x sweep, pin, y sweep, pin, z sweep, pin.  Asynchronous on
- * the solve's stream.  A grid that stays in the L2 and whose lines fit in shared
- * memory (without internalization tracking, timing, partitioned lines or launch
- * settings of its own) runs up to 64 steps per launch; elsewhere runs
+ * the solve's stream.  A grid that stays in the L2, whose lines fit in shared
+ * memory and which leaves room for others or keeps the SMs busy (without
+ * internalization tracking, timing, partitioned lines or launch settings of its
+ * own) runs up to 64 steps per launch; elsewhere runs
  * of more than 16 steps replay a captured CUDA graph of 16 steps (recaptured
  * when the agents, tracking or launch settings change), unless per-step timing
  * is on or the caller is capturing the solve's stream itself; the results are

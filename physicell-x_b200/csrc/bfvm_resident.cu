@@ -20,7 +20,7 @@
 // 32 dependent cycles and the loads about them), back 1,100-1,300, the x rows
 // out 1,900, then the barrier 2,500-3,400 (two memory latencies and what the
 // CTAs differ by); the sources 900.  Against a launch per stage, us per step in
-// calls of 10 steps (of 64, where those replay a captured graph):
+// calls of 10 steps (of 64, where those replay a captured graph), one solve alone:
 //   20x20x20x2    FP64 26.3 -> 12.7 (16.7 -> 10.8)
 //   50x50x50x2    FP64 32.3 -> 15.5 (24.8 -> 13.9)  FP32 34.2 -> 15.3 (25.5 -> 13.5)
 //   64x64x64x8    FP64 38.6 -> 22.9 (29.7 -> 21.2), seven warps to an SM
@@ -1001,8 +1001,8 @@ template <typename T>
 bool resident_plan(const bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, bool two_d, bool many, int sms,
                    ResidentPlan* plan, long long* tiles, size_t* smem) {
   const SweepConfig& g = c->cfg;
-  if (c->timing || c->sources_set || (p.line_off != nullptr && c->track) || c->sub_streams != 1 || g.persistent != 1 || g.tmem != 1 ||
-      g.x_lines != 32 || g.yz_tile != 32)
+  if (c->timing || c->sources_set || (p.line_off != nullptr && c->track) || c->sub_streams != 1 ||
+      g.persistent != 1 || g.tmem != 1 || g.x_lines != 32 || g.yz_tile != 32)
     return false;
   if (!two_d && (partitioned<T, 1>(c, p) || partitioned<T, 2>(c, p))) return false;  // (serial lines here)
   const int n[3] = {c->nx, c->ny, c->nz}, S = c->S;
@@ -1103,32 +1103,48 @@ bool resident_wins(const bfvm_ctx* c, const ResidentPlan& pl) {
 
 // And for a solve that has the GPU to itself or shares it with others on
 // streams of their own, which a launch per stage leaves more room for.  us per
-// call, FP32 unless stated, a launch per stage -> this, alone and three at once:
+// call, a launch per stage -> this, alone and three at once:
 //   two CTAs to an SM: 50x50x50x2 FP64 1 step 32 -> 22 and 22 -> 10, 10 steps
 //     309 -> 147 and 153 -> 54; 33x47x61x3 FP64 10 steps 319 -> 149 and 152 -> 80
-//   one: 64x64x64x8 (seven warps an SM) 1 step 37 -> 28 and 19 -> 24, 4 steps
-//     143 -> 78 and 71 -> 75, 10 steps 354 -> 178 and 177 -> 174
-//   ten steps by how busy the warps' lanes are: 58x25x184x2 (0.25: 736 y tiles,
-//     100 z tiles) 391 -> 186 and 163 -> 182, 150x24x24x3 FP64 (0.25) 370 -> 176
-//     and 153 -> 174, 120x30x30x6 FP64 (0.46) 370 -> 175 and 161 -> 172,
-//     33x47x61x7 FP64 (0.50) 339 -> 173 and 170 -> 169; several tiles per warp:
-//     58x25x184x4 (0.46) 411 -> 222 and 182 -> 218, 100x100x100x3 FP64 (0.63)
-//     702 -> 419 and 402 -> 416, 200x200x200x1 FP64 (0.70) 1357 -> 1027 and 1111
-//     -> 1034, 128x128x128x4 (0.99) 771 -> 511 and 547 -> 511
+//   one: 64x64x64x8 FP32 (seven warps an SM) 1 step 37 -> 28 and 19 -> 24, 4 steps
+//     143 -> 78 and 71 -> 75
 //   with agents in 1 voxel of 17: 100x100x100x3 FP64 702 -> 499 and 437 -> 502,
 //     120x30x30x6 370 -> 205 and 163 -> 203: a tile takes them 32 at a time, a
 //     launch of its own with all threads
-// so runs that leave no room for another come with four steps and more, agents
-// in less than 1 voxel of 32, and lanes that are busy.
+// A run that fills the SMs is 1.3 to 2.2 times as fast alone, but others wait for
+// it, and its idle warps are theirs.  Per call and solve, three at once:
+//   10 steps, a tile per warp, FP32: 50x50x50x8 176 -> 160, 64x64x64x8 191 -> 178,
+//     100x100x100x2 236 -> 230, 128x128x128x2 275 -> 280, 160x160x160x1 313 -> 330;
+//     FP64: 50x50x50x8 184 -> 175, 64x64x64x8 211 -> 225, 80x80x80x4 234 -> 250,
+//     100x100x100x2 256 -> 261, 112x112x112x2 283 -> 304; but fewer warps or lines
+//     too short to hide the barriers in: 96x96x96x2 FP64 (four) 198 -> 234,
+//     60x60x60x6 FP32 (five) 0.93 of it, 32x32x32x24 (lines of 32) 0.86; and lanes
+//     or warps that idle: 58x25x184x2 FP32 (busy 0.25) 163 -> 182, 120x60x60x4
+//     (0.65) 189 -> 201
+//   20 steps, where a launch per stage replays its graph: FP32 50x50x50x8 293 ->
+//     312, 100x100x100x2 395 -> 454; FP64 97x102x98x2 464 -> 525, 64x64x64x6 323 ->
+//     387, 96x96x96x3 465 -> 549: FP64 gives way
+//   several tiles per warp, either: FP64 50x50x50x20 (2.5 million values) 1.14 times
+//     as fast, 64x64x64x12 0.95, 128x128x128x2 474 -> 479, 160x160x160x1 552 -> 533,
+//     128x128x128x4 1025 -> 755, but 120x60x60x4 (1.7 million) 216 -> 280, 128x64x64x4
+//     0.79 and 256x128x128x1 (busy 0.69) 0.91; FP32 64x64x64x16 0.89, 256x128x128x1
+//     0.84, 200x200x100x1 355 -> 397: gives way; from 6 million values on, past the L2
+//     three at once, all of them 0.95 to 1.7 (busy 0.70 and more; 100x100x100x3 FP64,
+//     0.63, 402 -> 416)
+//   planes, few tiles of long lines: 600x600x4 FP64 0.76, 400x700x4 0.62: gives way
 template <typename T>
-bool resident_shares(const bfvm_ctx* c, const SweepParams<T>& p, const long long* tiles, long long warps, int nsteps,
-                     double busy) {
-  const long long voxels = static_cast<long long>(c->nx) * c->ny * c->nz;
-  if (nsteps < 4 || (p.line_off != nullptr && 32ll * c->n_agents > voxels)) return false;
+bool resident_shares(const bfvm_ctx* c, const SweepParams<T>& p, const long long* tiles, int sms, long long warps,
+                     bool two_d, int nsteps) {
+  const long long voxels = static_cast<long long>(c->nx) * c->ny * c->nz, values = voxels * c->S;
+  if (two_d || nsteps < 4 || (p.line_off != nullptr && 32ll * c->n_agents > voxels)) return false;
   const long long n[3] = {c->nx, c->ny, c->nz};
+  const long long most = std::max(tiles[0], std::max(tiles[1], tiles[2])), line = std::max(n[0], std::max(n[1], n[2]));
   double slots = 0;  // values that the warps' lanes could take meanwhile
   for (int a = 0; a < 3; ++a) slots += static_cast<double>((tiles[a] + warps - 1) / warps * warps) * 32 * n[a];
-  return 3.0 * voxels * c->S >= busy * slots;
+  const double busy = 3.0 * values / slots;
+  if (values >= 6000000) return busy >= 0.65;
+  if (most <= warps) return warps > 5ll * sms && busy >= 0.67 && line >= 40 && (sizeof(T) == 4 || nsteps <= 16);
+  return sizeof(T) == 8 && values >= 2500000 && busy >= 0.75;
 }
 
 int sm_count(int device, int* sms) {
@@ -1171,8 +1187,8 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
     }
     // whether another such run finds room beside this one: 227 KB and eight warps an SM
     const long long per_sm = std::min<long long>(kSmemMax / smem, kResidentWarps / std::max(pl.warps, threads / 32));
-    if (2 * grid > per_sm * sms && !resident_shares(c, p, tiles, static_cast<long long>(grid) * pl.warps, nsteps, 0.5))
-      return BFVM_OK;
+    const long long all = static_cast<long long>(grid) * pl.warps;
+    if (2 * grid > per_sm * sms && !resident_shares(c, p, tiles, sms, all, two_d, nsteps)) return BFVM_OK;
     pl.crowd = resident_crowd(c, p, static_cast<long long>(grid) * threads);
     int blocks = 0;
     BFVM_CUDA(persistent_grid(resident_kernel<T>, smem, grid, &blocks, threads));
@@ -1192,7 +1208,7 @@ int run_resident(bfvm_ctx* c, const SweepParams<T>& p, const NodeLines& nodes, b
     const long long all = static_cast<long long>(grid) * pl.warps, rounds = (most + all - 1) / all;
     // no more warps than that many rounds need
     const int warps = static_cast<int>((most + grid * rounds - 1) / (grid * rounds));
-    if (!resident_wins<T>(c, pl) || !resident_shares(c, p, tiles, static_cast<long long>(grid) * warps, nsteps, 0.65))
+    if (!resident_wins<T>(c, pl) || !resident_shares(c, p, tiles, sms, static_cast<long long>(grid) * warps, false, nsteps))
       return BFVM_OK;
     smem -= static_cast<size_t>(pl.warps - warps) * pl.warp_bytes;
     pl.warps = warps;

@@ -106,3 +106,28 @@ def test_batch_members_side_by_side_are_one_launch(precision):
         batch.close()
         for me in mes:
             me.close()
+
+
+# Runs that fill the SMs: a tile per warp and several, with enough to do; and those
+# that other streams' solves would wait for: few warps, short lines, idle lanes,
+# few values, FP64 in calls that replay a graph, dense agents, a call of 3 steps;
+# and planes.
+@pytest.mark.parametrize("shape,agents,steps,one", [
+    ((50, 50, 50, 8), 300, 10, True), ((50, 50, 50, 8), 300, 20, "fp32"), ((50, 50, 50, 8), 300, 3, False),
+    ((50, 50, 50, 8), 9000, 10, False), ((128, 100, 100, 2), 300, 10, True), ((60, 60, 60, 6), 300, 10, False),
+    ((32, 32, 32, 24), 300, 10, False), ((128, 64, 64, 4), 300, 10, "fp32"), ((64, 64, 64, 16), 300, 10, "fp64"),
+    ((128, 128, 128, 2), 300, 20, True), ((129, 127, 128, 3), 300, 20, True), ((40, 36, 300, 4), 300, 10, False),
+    ((600, 400, 1, 4), 300, 10, "fp32"), ((100, 130, 1, 4), 300, 10, True)])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_runs_that_fill_the_gpu(shape, agents, steps, one, precision):
+    nx, ny, nz, S = shape
+    wl = W.small_random(steps + nx, nx=nx, ny=ny, nz=nz, S=S, n_agents=agents, steps=1)
+    me, solo = (Microenvironment.from_workload(wl, precision=precision) for _ in range(2))
+    solo.set_sweep_tmem(0)
+    step = "simulate_diffusion_decay" + ("_2d" if nz == 1 else "")
+    launches = _launches(lambda: getattr(me, step)(steps, sources=True))
+    assert launches == (1 if one in (True, precision) else (3 if nz == 1 else 4) * steps)
+    getattr(solo, step)(steps, sources=True)
+    assert np.array_equal(me.download_field(), solo.download_field())
+    me.close()
+    solo.close()

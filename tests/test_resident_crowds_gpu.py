@@ -33,7 +33,7 @@ def _crowd(shape, n, seed):
 
 # One tile per warp, several, and a plane; as many agents as a tile still takes
 # and one more, and many of them.
-SHAPES = [(40, 36, 30, 2), (64, 64, 80, 8), (90, 127, 1, 2)]
+SHAPES = [(40, 36, 30, 2), (64, 64, 110, 8), (90, 127, 1, 2)]
 
 
 @pytest.mark.parametrize("shape", SHAPES)

@@ -47,7 +47,7 @@ def _expect(wl, precision, n):
 
 
 # One tile per warp, several, and a plane.
-@pytest.mark.parametrize("shape", [(50, 50, 50, 2), (64, 64, 96, 6), (90, 127, 1, 2)])
+@pytest.mark.parametrize("shape", [(50, 50, 50, 2), (128, 128, 128, 3), (90, 127, 1, 2)])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_a_barrier_that_gives_up_leaves_the_solve_usable(shape, precision):
     """With a limit of 1 us the CTAs that wait for the stack's give up, in both
